@@ -393,7 +393,7 @@ __device__ __forceinline__ int recon_learned(const Grid<float> &G, uint32_t *sW,
 // (weno_all).  There are F x LINES lines of W+2 cells (positions 0..W+1,
 // cells -1..W); the faces of a line read both edges of the W inner cells, the
 // right edge of position 0 and the left edge of position W+1.  Inner cells go
-// two per thread and iteration (weno9_edges2, recon_packed_inner); the two
+// two per thread and iteration (weno9_edges, recon_packed_inner); the two
 // halo cells of a line go together through the one-edge form
 // (weno9_outer_edges2, recon_outer_pair), which skips the two edges nobody
 // reads.  Per stencil and edge the bits are those of weno9_edges.
@@ -430,7 +430,7 @@ __device__ __forceinline__ void recon_packed_inner(Mask mask, Vals vals, Store s
       float2 s2[9], qL, qR;
 #pragma unroll
       for (int m = 0; m < 9; m++) s2[m] = make_float2(a[m], b[m]);
-      weno9_edges2(s2, qL, qR, bool2{!ax, !ax}, bool2{il, il}, bool2{ir, ir});
+      weno9_edges(s2, qL, qR, bool2{!ax, !ax}, bool2{il, il}, bool2{ir, ir});
       store(f, line, pos, qL.x, qR.x);
       store(f + 1, line, pos, qL.y, qR.y);
     }
@@ -467,7 +467,7 @@ __device__ __forceinline__ void recon_packed_inner(Mask mask, Vals vals, Store s
       float2 s2[9], qL, qR;
 #pragma unroll
       for (int m = 0; m < 9; m++) s2[m] = make_float2(a[m], b[m]);
-      weno9_edges2(s2, qL, qR, bool2{!xa, !xb}, bool2{((ia >> 3) & 1u) != 0, ((ib >> 3) & 1u) != 0},
+      weno9_edges(s2, qL, qR, bool2{!xa, !xb}, bool2{((ia >> 3) & 1u) != 0, ((ib >> 3) & 1u) != 0},
                    bool2{((ia >> 5) & 1u) != 0, ((ib >> 5) & 1u) != 0});
       store(fa, la, pa, qL.x, qR.x);
       if (two) store(fb, lb, pb, qL.y, qR.y);
@@ -1109,7 +1109,7 @@ __global__ void __launch_bounds__(TX *TY, LEARNED ? PU_LEARNED_Z_MIN_BLOCKS : (s
 #pragma unroll
               for (int m = 0; m < 9; m++) s2[m] = make_float2(a[m], b[m]);
               const bool il = (imm >> 3) & 1u, ir = (imm >> 5) & 1u;
-              weno9_edges2(s2, qL, qR, bool2{!any10, !any10}, bool2{il, il}, bool2{ir, ir});
+              weno9_edges(s2, qL, qR, bool2{!any10, !any10}, bool2{il, il}, bool2{ir, ir});
               eL[f * NT + tid] = qL.x;
               eL[(f + 1) * NT + tid] = qL.y;
               eRc[f * NT] = qR.x;

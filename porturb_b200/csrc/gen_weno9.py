@@ -17,6 +17,19 @@ form that needs fewer operations per stencil:
       TV_k = sum_r D_r * y_r^2,   y_r = d_{k+r} + sum_{c>r} L[c][r] d_{k+c}
   which costs 6 multiply-adds for the y's and 4 for the sum, and is a sum of
   non-negative terms (no cancellation in the final sum).
+* Difference form (the limiter's own arithmetic).  With the nested differences
+  d (first) .. e4 (fourth) of the stencil, each window's polynomial about the
+  centre cell is described by e4 and three numbers (difference_form below):
+      A    half its third central difference at the centre cell,
+      sec  its second difference there (even part),
+      h    its central difference there, s(+1) - s(-1) (odd part).
+  With W = SW sec + CW e4 and O = OS h + CO A
+      4 TV / CA = O^2 + W^2 + A^2 + C4 e4^2
+  with the same constants for every window, and the edge values are
+      q_R, q_L = s_4 + OUT ((W + CX e4) +- SO O),
+  so a window's TV and both its edge values share their linear forms.  Each
+  window reads only its own five cells, as the direct form does: a window
+  beside a jump carries none of the jump's rounding.
 * Edge values.  Each window polynomial's value at the cell's left and right
   edge (WenoLimiter.h:382-426) is s_4 plus a linear form in the window's four
   differences.
@@ -98,6 +111,23 @@ def ldl(B):
     return L, D
 
 
+def difference_form(s):
+    """(e4, A, h, sec) of the five windows of a 9-cell stencil, each at the
+    centre cell, from that window's own differences."""
+    d = [s[m + 1] - s[m] for m in range(8)]
+    e2 = [d[m + 1] - d[m] for m in range(7)]
+    e3 = [e2[m + 1] - e2[m] for m in range(6)]
+    e4 = [e3[m + 1] - e3[m] for m in range(5)]
+    half = Fr(1, 2)
+    A = [e3[1] + 3 * half * e4[0], e3[2] + half * e4[1], e3[2] + half * e4[2], e3[3] - half * e4[3],
+         e3[4] - 3 * half * e4[4]]
+    lo = e2[2] + (e3[1] + e4[0])      # windows 0 and 4 extend their quartic to the centre's neighbour
+    hi = e2[4] - (e3[4] - e4[4])
+    sec = [lo, e2[3], e2[3], e2[3], hi]
+    h = [2 * d[3] + lo] + 3 * [d[3] + d[4]] + [2 * d[4] - hi]
+    return e4, A, h, sec
+
+
 def lit(v):
     return repr(float(v))
 
@@ -149,6 +179,15 @@ def main():
                 for m in range(j, 4):
                     f[m] -= e[j]
         s2e.append(f)
+    # Constants of the difference form: TV(a) = (a1 + a3/4)^2 + ca a3^2 +
+    # c2 (a2 + beta a4)^2 + c4 a4^2 with a4 = e4/24, a3 = A/6, a2 = sec/2 - e4/16, a1 = h/2 - 5/24 A.
+    beta = Q[2][4] / Q[2][2]
+    ca, c4 = Q[3][3] - Q[1][3] ** 2, Q[4][4] - Q[2][4] ** 2 / Q[2][2]
+    assert Q[1][1] == 1 and Q[1][3] == Fr(1, 4)
+    CA, C4, SW2 = 4 * ca / 36, 4 * c4 / 576, Q[2][2]
+    cw4 = beta / 12 - Fr(1, 8)        # W / SW = sec + cw4 e4 = 2 (a2 + beta a4)
+    cx4 = -Fr(1, 10) - cw4            # 12 * (a2/6 + a4/20) = sec - e4/10 = W / SW + cx4 e4
+    SW, OS = float(SW2 / CA) ** 0.5, float(1 / CA) ** 0.5
     # Verify the reformulation against the direct forms on random rationals.
     import random
     rnd = random.Random(1)
@@ -163,6 +202,11 @@ def main():
             assert sum(chol_D[k][r] * y[r] ** 2 for r in range(4)) == tv_direct
             el = sum(a[dd] * Fr(-1, 2) ** dd for dd in range(5))
             assert el == s[4] + sum(lin_l[k][m] * d[k + m] for m in range(4))
+            er = sum(a[dd] * Fr(1, 2) ** dd for dd in range(5))
+            e4, A, h, sec = (f[k] for f in difference_form(s))
+            W, O = sec + cw4 * e4, h - A / 3
+            assert O ** 2 + SW2 * W ** 2 + CA * A ** 2 + C4 * e4 ** 2 == 4 * tv_direct
+            assert W + cx4 * e4 + 3 * O == 12 * (er - s[4]) and W + cx4 * e4 - 3 * O == 12 * (el - s[4])
 
     w("// Generated by gen_weno9.py from exact rational arithmetic. Do not edit.\n")
     w("// Order-9 WENO tables in stencil-difference form; see gen_weno9.py.\n")
@@ -182,6 +226,11 @@ def main():
         for k in range(5):
             w("  {%s},\n" % ", ".join(lit(v) for v in tab[k]))
         w("};\n")
+    w("// Difference form: 4 TV_k / DF_CA = O^2 + W^2 + A^2 + DF_C4 e4^2, W = DF_SW sec + DF_CW e4,\n")
+    w("// O = DF_OS h + DF_CO A; edge values s_4 + DF_OUT ((W + DF_CX e4) -+ DF_SO O).\n")
+    for nm, v in (("CA", CA), ("SW", SW), ("CW", SW * float(cw4)), ("CX", SW * float(cx4)), ("OS", OS), ("CO", -OS / 3),
+                  ("C4", C4 / CA), ("SO", 3 * SW / OS), ("OUT", 1 / (12 * SW))):
+        w("__device__ constexpr double DF_%s = %s;\n" % (nm, lit(v)))
     w("__device__ constexpr double IDEAL_L[5] = {%s};\n" % ", ".join(lit(v) for v in ideal_l))
     w("__device__ constexpr double IDEAL_R[5] = {%s};\n" % ", ".join(lit(v) for v in ideal_r))
     w("// Nine-cell linear edges minus s_4, over d_0..d_7.\n")

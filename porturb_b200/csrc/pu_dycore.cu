@@ -424,7 +424,7 @@ __global__ void k_weno9_eval(const float *__restrict__ s, const unsigned char *_
         ir{(fa & 4u) != 0, (fb & 4u) != 0};
     if constexpr (VARIANT == 1) {
       float2 L, R;
-      pu::weno9_edges2(st, L, R, mp, il, ir);
+      pu::weno9_edges(st, L, R, mp, il, ir);
       qL[a] = L.x;
       qR[a] = R.x;
       if (b < n) {

@@ -208,15 +208,27 @@ __device__ __forceinline__ void issue(uint32_t taddr, const uint32_t *ahi, const
   mma_tf32(taddr, ah, bh, 1u);
 }
 
+// (convexify, WenoLimiter.h:30-34)
+__device__ __forceinline__ void convexify5(float (&w)[5]) {
+  const float tot = sum5(w);
+  if (tot > 1.e-20f) {
+    const float r = fast_rcp(tot);
+#pragma unroll
+    for (int k = 0; k < 5; k++) w[k] *= r;
+  }
+}
+
 // Edge value from the linear forms of one edge and the shared reciprocals,
-// as weno9_edge does from the differences.
+// as weno9_edge does from the windows.
 template <bool LEFT>
 __device__ __forceinline__ float edge_from_lin(const float (&lin)[5], float s4, const float (&rk)[5], bool do_map) {
   using namespace pu_weno9;
   float w[5];
 #pragma unroll
   for (int k = 0; k < 5; k++) w[k] = float(LEFT ? IDEAL_L[k] : IDEAL_R[k]) * rk[k];
-  normalize5(w);
+  const float rs = fast_rcp(sum5(w));
+#pragma unroll
+  for (int k = 0; k < 5; k++) w[k] *= rs;
   float r = 1.f;
   if (do_map) {
 #pragma unroll

@@ -9,10 +9,19 @@
 //   3. per edge: w_k = ideal_k / (TV_k^2 + 1e-20), normalise, optionally
 //      apply map_rs (k=6, m=3, s=2000; WenoLimiter.h:75-82) and normalise
 //      again, then the weighted sub-stencil edge values (WenoLimiter.h:382-426).
-// The arithmetic is rearranged (see gen_weno9.py): stencil differences, an
-// LDL^T form of TV, edge values as s_4 plus linear forms, one reciprocal
-// shared by both edges for each 1/(TV_k^2+1e-20), and the normalisation
-// after map_rs applied once to the weighted sum instead of to each weight.
+// The arithmetic is rearranged (difference form, see gen_weno9.py): nested
+// stencil differences, per window three linear forms that give both its TV
+// and its two edge values, one reciprocal shared by both edges for each
+// 1/(TV_k^2+1e-20), and the normalisation after map_rs applied once to the
+// weighted sum instead of to each weight.
+//
+// The stencil kernels are bound by the FP32 multiply-add pipe, so the count
+// of these operations is what the limiter costs: ~256 per stencil (both
+// edges) against ~280 for the earlier form (an LDL^T factorisation of each
+// window's TV and separate edge formulas, 118 operations up to the TVs and
+// edge values where this one takes 94), and ~25 distinct constants instead
+// of ~100: the 256x256x128 boundary layer 6.53 -> 6.14 ms per step, the
+// 512x512x128 urban canopy 24.2 -> 22.6 ms, the FP64 build 9 % faster.
 // In FP32 the reciprocals use rcp.approx.ftz; every operand is a normal
 // number there: TV_k^2+1e-20 >= 1e-20, the normalisation sums exceed 1e-20
 // on the branch that divides (the weight sums always), and the map_rs
@@ -33,267 +42,234 @@ __device__ __forceinline__ float fast_rcp<float>(float x) {
   return r;
 }
 
-template <class R>
-__device__ __forceinline__ void convexify5(R (&w)[5]) {
-  R tot = w[0] + w[1] + w[2] + w[3] + w[4];
-  if (tot > R(1.e-20)) {
-    R r = fast_rcp(tot);
-#pragma unroll
-    for (int k = 0; k < 5; k++) w[k] *= r;
-  }
-}
-
-// convexify of the ideal-weighted reciprocals, whose sum always passes the
-// reference's test (> 1e-20): rk_k = 1/(TV_k^2 + 1e-20) is at least
-// 1/(1 + 1e-20) when the TV were normalised (each is then at most 1 up to a
-// rounding) and far above 1 when they were not (sum of TV <= 1e-20), so the
-// sum is at least the sum of the ideal weights, 1.
-template <class R>
-__device__ __forceinline__ void normalize5(R (&w)[5]) {
-  const R r = fast_rcp(w[0] + w[1] + w[2] + w[3] + w[4]);
-#pragma unroll
-  for (int k = 0; k < 5; k++) w[k] *= r;
-}
-
-// One edge: weights from the shared reciprocals rk = 1/(TV_k^2 + 1e-20).
-// After map_rs the second convexify is folded into the edge value: the
-// weighted sum of the sub-stencil edges is taken with the mapped weights
-// m_k and scaled once by 1/sum(m) (the reference scales each weight).  The
-// test of that convexify always passes: each m_k >= min(w_k, ideal_k) >= 0,
-// and the k with w_k >= 1/5 gives m_k >= min_k ideal_k = 1/126.
-template <class R, bool LEFT>
-__device__ __forceinline__ R weno9_edge(const R (&d)[8], R s4, const R (&rk)[5], bool do_map) {
-  using namespace pu_weno9;
-  R w[5];
-#pragma unroll
-  for (int k = 0; k < 5; k++) w[k] = R(LEFT ? IDEAL_L[k] : IDEAL_R[k]) * rk[k];
-  normalize5(w);
-  R r = R(1);
-  if (do_map) {
-#pragma unroll
-    for (int k = 0; k < 5; k++) {
-      const R dk = R(LEFT ? IDEAL_L[k] : IDEAL_R[k]);
-      R t = w[k] - dk;
-      R t2 = t * t;
-      R t6 = t2 * t2 * t2;
-      R u = fma(-w[k], w[k], w[k]);   // w (1 - w)
-      R u3 = u * u * u;
-      R den = fma(R(2000.), u3, t6);
-      w[k] = fma(t6 * t, fast_rcp(den), dk);
-    }
-    r = fast_rcp(w[0] + w[1] + w[2] + w[3] + w[4]);
-  }
-  R acc = R(0);
-#pragma unroll
-  for (int k = 0; k < 5; k++) {
-    R lin = R(LEFT ? LIN_L[k][0] : LIN_R[k][0]) * d[k];
-#pragma unroll
-    for (int m = 1; m < 4; m++) lin = fma(R(LEFT ? LIN_L[k][m] : LIN_R[k][m]), d[k + m], lin);
-    acc = fma(w[k], lin, acc);
-  }
-  return fma(acc, r, s4);
-}
-
-template <class R>
-__device__ __forceinline__ void weno9_edges(const R (&s)[9], R &qL, R &qR, bool do_map, bool imm_L, bool imm_R) {
-  using namespace pu_weno9;
-  R d[8];
-#pragma unroll
-  for (int m = 0; m < 8; m++) d[m] = s[m + 1] - s[m];
-  R tv[5];
-#pragma unroll
-  for (int k = 0; k < 5; k++) {
-    R y3 = d[k + 3];
-    R y2 = fma(R(TV_L[k][3][2]), d[k + 3], d[k + 2]);
-    R y1 = fma(R(TV_L[k][3][1]), d[k + 3], fma(R(TV_L[k][2][1]), d[k + 2], d[k + 1]));
-    R y0 = fma(R(TV_L[k][3][0]), d[k + 3], fma(R(TV_L[k][2][0]), d[k + 2], fma(R(TV_L[k][1][0]), d[k + 1], d[k])));
-    R t = R(TV_D[k][3]) * y3 * y3;
-    t = fma(R(TV_D[k][2]) * y2, y2, t);
-    t = fma(R(TV_D[k][1]) * y1, y1, t);
-    tv[k] = fma(R(TV_D[k][0]) * y0, y0, t);
-  }
-  convexify5(tv);
-  if (imm_L || imm_R) {
-    R mx = fmax(fmax(fmax(fmax(tv[0], tv[1]), tv[2]), tv[3]), tv[4]);
-    if (imm_L) tv[4] = mx;
-    if (imm_R) tv[0] = mx;
-  }
-  R rk[5];
-#pragma unroll
-  for (int k = 0; k < 5; k++) rk[k] = fast_rcp(fma(tv[k], tv[k], R(1.e-20)));
-  qL = weno9_edge<R, true>(d, s[4], rk, do_map);
-  qR = weno9_edge<R, false>(d, s[4], rk, do_map);
-}
-
 // ---------------------------------------------------------------------------
-// Two stencils at once with packed FP32 arithmetic (FFMA2/FADD2/FMUL2 on
-// sm_100): the same operations in the same order as weno9_edges<float>, per
-// component, so each component's result is bit-identical to the scalar
-// limiter's.  Halves the issue slots of the FP32 work; reciprocals stay
-// scalar (rcp.approx.ftz per component).  Branches of the scalar form
-// become per-component selects (a multiply by exactly 1 where the scalar
-// form skips the normalisation).
+// Arithmetic of one stencil (float, double) or of two at once (float2, the
+// packed FFMA2/FADD2/FMUL2 of sm_100).  Every operation is rounded by itself
+// and the limiter below is written once over them, so each lane of the packed
+// form gives the scalar form's bits.  A difference in the packed form is
+// fma(b, -1, a), which is one operation whether or not the packed add takes a
+// negated operand, with the same rounding.
 // ---------------------------------------------------------------------------
 struct bool2 {
   bool x, y;
 };
-__device__ __forceinline__ float2 f2(float a) { return make_float2(a, a); }
-__device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
-__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __fadd2_rn(a, make_float2(-b.x, -b.y)); }
-__device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
-__device__ __forceinline__ float2 rcp2(float2 a) { return make_float2(fast_rcp(a.x), fast_rcp(a.y)); }
+template <class V>
+struct Arith;
 
-__device__ __forceinline__ void convexify5x2(float2 (&w)[5]) {
-  const float2 tot = add2(add2(add2(add2(w[0], w[1]), w[2]), w[3]), w[4]);
-  const float2 r = make_float2(tot.x > 1.e-20f ? fast_rcp(tot.x) : 1.f, tot.y > 1.e-20f ? fast_rcp(tot.y) : 1.f);
-#pragma unroll
-  for (int k = 0; k < 5; k++) w[k] = mul2(w[k], r);
+template <>
+struct Arith<float> {
+  using V = float;
+  using B = bool;
+  static __device__ __forceinline__ V c(double a) { return float(a); }
+  static __device__ __forceinline__ V c2(double, double b) { return float(b); }
+  static __device__ __forceinline__ V add(V a, V b) { return __fadd_rn(a, b); }
+  static __device__ __forceinline__ V sub(V a, V b) { return __fsub_rn(a, b); }
+  static __device__ __forceinline__ V mul(V a, V b) { return __fmul_rn(a, b); }
+  static __device__ __forceinline__ V fma(V a, V b, V x) { return fmaf(a, b, x); }
+  static __device__ __forceinline__ V rcp(V a) { return fast_rcp(a); }
+  static __device__ __forceinline__ V neg(V a) { return -a; }
+  static __device__ __forceinline__ V max(V a, V b) { return fmaxf(a, b); }
+  static __device__ __forceinline__ B gt(V a, float b) { return a > b; }
+  static __device__ __forceinline__ V sel(B q, V a, V b) { return q ? a : b; }
+  static __device__ __forceinline__ bool any(B q) { return q; }
+};
+
+template <>
+struct Arith<double> {
+  using V = double;
+  using B = bool;
+  static __device__ __forceinline__ V c(double a) { return a; }
+  static __device__ __forceinline__ V c2(double, double b) { return b; }
+  static __device__ __forceinline__ V add(V a, V b) { return __dadd_rn(a, b); }
+  static __device__ __forceinline__ V sub(V a, V b) { return __dsub_rn(a, b); }
+  static __device__ __forceinline__ V mul(V a, V b) { return __dmul_rn(a, b); }
+  static __device__ __forceinline__ V fma(V a, V b, V x) { return ::fma(a, b, x); }
+  static __device__ __forceinline__ V rcp(V a) { return fast_rcp(a); }
+  static __device__ __forceinline__ V neg(V a) { return -a; }
+  static __device__ __forceinline__ V max(V a, V b) { return fmax(a, b); }
+  static __device__ __forceinline__ B gt(V a, double b) { return a > b; }
+  static __device__ __forceinline__ V sel(B q, V a, V b) { return q ? a : b; }
+  static __device__ __forceinline__ bool any(B q) { return q; }
+};
+
+template <>
+struct Arith<float2> {
+  using V = float2;
+  using B = bool2;
+  static __device__ __forceinline__ V c(double a) { return make_float2(float(a), float(a)); }
+  static __device__ __forceinline__ V c2(double a, double b) { return make_float2(float(a), float(b)); }
+  static __device__ __forceinline__ V add(V a, V b) { return __fadd2_rn(a, b); }
+  static __device__ __forceinline__ V sub(V a, V b) { return __ffma2_rn(b, make_float2(-1.f, -1.f), a); }
+  static __device__ __forceinline__ V mul(V a, V b) { return __fmul2_rn(a, b); }
+  static __device__ __forceinline__ V fma(V a, V b, V x) { return __ffma2_rn(a, b, x); }
+  static __device__ __forceinline__ V rcp(V a) { return make_float2(fast_rcp(a.x), fast_rcp(a.y)); }
+  static __device__ __forceinline__ V neg(V a) { return make_float2(-a.x, -a.y); }
+  static __device__ __forceinline__ V max(V a, V b) { return make_float2(fmaxf(a.x, b.x), fmaxf(a.y, b.y)); }
+  static __device__ __forceinline__ B gt(V a, float b) { return bool2{a.x > b, a.y > b}; }
+  static __device__ __forceinline__ V sel(B q, V a, V b) { return make_float2(q.x ? a.x : b.x, q.y ? a.y : b.y); }
+  static __device__ __forceinline__ bool any(B q) { return q.x || q.y; }
+};
+
+template <class V>
+__device__ __forceinline__ V sum5(const V (&w)[5]) {
+  using A = Arith<V>;
+  return A::add(A::add(A::add(A::add(w[0], w[1]), w[2]), w[3]), w[4]);
 }
 
-__device__ __forceinline__ void normalize5x2(float2 (&w)[5]) {
-  const float2 tot = add2(add2(add2(add2(w[0], w[1]), w[2]), w[3]), w[4]);
-  const float2 r = rcp2(tot);
-#pragma unroll
-  for (int k = 0; k < 5; k++) w[k] = mul2(w[k], r);
-}
-
-// Per-lane constants of one edge: SIDE 0 the left edge in both lanes, 1 the
-// right edge in both, 2 the right edge in lane x and the left edge in lane y.
-template <int SIDE>
-__device__ __forceinline__ float2 ideal2(int k) {
+// The five windows of a stencil in difference form: X and O, whose sum and
+// difference (O scaled by DF_SO) are 1/DF_OUT times the window's right and
+// left edge value minus s_4, and tv = 4 TV / DF_CA.
+template <class V>
+__device__ __forceinline__ void weno9_windows(const V (&s)[9], V (&X)[5], V (&O)[5], V (&tv)[5]) {
   using namespace pu_weno9;
-  return SIDE == 0 ? f2(float(IDEAL_L[k])) : SIDE == 1 ? f2(float(IDEAL_R[k]))
-                                                       : make_float2(float(IDEAL_R[k]), float(IDEAL_L[k]));
-}
-template <int SIDE>
-__device__ __forceinline__ float2 lin2(int k, int m) {
-  using namespace pu_weno9;
-  return SIDE == 0 ? f2(float(LIN_L[k][m])) : SIDE == 1 ? f2(float(LIN_R[k][m]))
-                                                        : make_float2(float(LIN_R[k][m]), float(LIN_L[k][m]));
+  using A = Arith<V>;
+  V d[8], e2[7], e3[6], e4[5];
+#pragma unroll
+  for (int m = 0; m < 8; m++) d[m] = A::sub(s[m + 1], s[m]);
+#pragma unroll
+  for (int m = 0; m < 7; m++) e2[m] = A::sub(d[m + 1], d[m]);
+#pragma unroll
+  for (int m = 0; m < 6; m++) e3[m] = A::sub(e2[m + 1], e2[m]);
+#pragma unroll
+  for (int m = 0; m < 5; m++) e4[m] = A::sub(e3[m + 1], e3[m]);
+  // Second and central first difference at the centre cell: windows 1 to 3
+  // hold the centre's neighbours, windows 0 and 4 extend their quartic by one.
+  const V lo = A::add(e2[2], A::add(e3[1], e4[0])), nhi = A::sub(A::sub(e3[4], e4[4]), e2[4]);
+  const V wm = A::mul(A::c(DF_SW), e2[3]);
+  const V hm = A::mul(A::c(DF_OS), A::add(d[3], d[4]));
+  const V w[5] = {A::mul(A::c(DF_SW), lo), wm, wm, wm, A::mul(A::c(-DF_SW), nhi)};
+  const V h[5] = {A::mul(A::c(DF_OS), A::fma(A::c(2.), d[3], lo)), hm, hm, hm,
+                  A::mul(A::c(DF_OS), A::fma(A::c(2.), d[4], nhi))};
+  const V a3[5] = {A::fma(A::c(1.5), e4[0], e3[1]), A::fma(A::c(.5), e4[1], e3[2]), A::fma(A::c(.5), e4[2], e3[2]),
+                   A::fma(A::c(-.5), e4[3], e3[3]), A::fma(A::c(-1.5), e4[4], e3[4])};
+#pragma unroll
+  for (int k = 0; k < 5; k++) {
+    const V W = A::fma(A::c(DF_CW), e4[k], w[k]);
+    O[k] = A::fma(A::c(DF_CO), a3[k], h[k]);
+    X[k] = A::fma(A::c(DF_CX), e4[k], W);
+    V t = A::mul(A::mul(A::c(DF_C4), e4[k]), e4[k]);
+    t = A::fma(a3[k], a3[k], t);
+    t = A::fma(W, W, t);
+    tv[k] = A::fma(O[k], O[k], t);
+  }
 }
 
-template <int SIDE>
-__device__ __forceinline__ float2 weno9_edge2(const float2 (&d)[8], float2 s4, const float2 (&rk)[5], bool2 do_map) {
-  float2 w[5];
+// From the windows' tv to the reciprocals rk = 1/(TV_k^2 + 1e-20) of the
+// normalised TVs (convexify: not normalised where the sum of the TVs is at
+// most 1e-20; TV_k^2 is then below 1e-38, and any fixed scale of tv leaves
+// rk at 1e20), with the immersed replacements (imm_L: TV_5 = max, imm_R:
+// TV_1 = max).
+template <class V>
+__device__ __forceinline__ void weno9_rk(V (&tv)[5], typename Arith<V>::B imm_L, typename Arith<V>::B imm_R,
+                                         V (&rk)[5]) {
+  using A = Arith<V>;
+  const V tot = sum5(tv);
+  const V r = A::sel(A::gt(tot, 4.e-20 / pu_weno9::DF_CA), A::rcp(tot), A::c(1.));
 #pragma unroll
-  for (int k = 0; k < 5; k++) w[k] = mul2(ideal2<SIDE>(k), rk[k]);
-  normalize5x2(w);
-  float2 r = f2(1.f);
-  if (do_map.x || do_map.y) {
-    float2 m[5];
+  for (int k = 0; k < 5; k++) tv[k] = A::mul(tv[k], r);
+  if (A::any(imm_L) || A::any(imm_R)) {
+    const V mx = A::max(A::max(A::max(A::max(tv[0], tv[1]), tv[2]), tv[3]), tv[4]);
+    tv[4] = A::sel(imm_L, mx, tv[4]);
+    tv[0] = A::sel(imm_R, mx, tv[0]);
+  }
+#pragma unroll
+  for (int k = 0; k < 5; k++) rk[k] = A::rcp(A::fma(tv[k], tv[k], A::c(1.e-20)));
+}
+
+// Per-lane constants of one edge: SIDE 0 the left edge, 1 the right edge, 2
+// (float2) the right edge in lane x and the left edge in lane y.
+template <class V, int SIDE>
+__device__ __forceinline__ V ideal_of(int k) {
+  using namespace pu_weno9;
+  return Arith<V>::c2(SIDE == 0 ? IDEAL_L[k] : IDEAL_R[k], SIDE == 1 ? IDEAL_R[k] : IDEAL_L[k]);
+}
+template <class V, int SIDE>
+__device__ __forceinline__ V odd_of() {
+  using namespace pu_weno9;
+  return Arith<V>::c2(SIDE == 0 ? -DF_SO : DF_SO, SIDE == 1 ? DF_SO : -DF_SO);
+}
+
+// The weights of one edge, negated: -w_k of the ideal-weighted normalised
+// reciprocals, or after map_rs the unnormalised -m_k, whose sum the caller
+// divides by (r: 1/sum(-m_k), or -1).  The signs spare every negated operand
+// in between: with n = -w,  n + d = -(w - d)  and  n n + n = -w (1 - w).
+// Both sums always pass the reference's test (> 1e-20): rk_k is at least
+// 1/(1 + 1e-20) when the TVs were normalised (each is then at most 1 up to a
+// rounding) and 1e20 when they were not, so the first is at least the sum of
+// the ideal weights, 1; each m_k >= min(w_k, ideal_k) >= 0, and the k with
+// w_k >= 1/5 gives m_k >= min_k ideal_k = 1/126.
+template <class V, int SIDE>
+__device__ __forceinline__ V weno9_neg_weights(const V (&rk)[5], typename Arith<V>::B do_map, V (&n)[5]) {
+  using A = Arith<V>;
+#pragma unroll
+  for (int k = 0; k < 5; k++) n[k] = A::mul(ideal_of<V, SIDE>(k), rk[k]);
+  const V rn = A::rcp(A::neg(sum5(n)));
+#pragma unroll
+  for (int k = 0; k < 5; k++) n[k] = A::mul(n[k], rn);
+  V r = A::c(-1.);
+  if (A::any(do_map)) {
+    V m[5];
 #pragma unroll
     for (int k = 0; k < 5; k++) {
-      const float2 dk = ideal2<SIDE>(k);
-      const float2 t = sub2(w[k], dk);
-      const float2 t2 = mul2(t, t);
-      const float2 t6 = mul2(mul2(t2, t2), t2);
-      const float2 u = fma2(make_float2(-w[k].x, -w[k].y), w[k], w[k]);
-      const float2 u3 = mul2(mul2(u, u), u);
-      const float2 den = fma2(f2(2000.f), u3, t6);
-      m[k] = fma2(mul2(t6, t), rcp2(den), dk);
+      const V dk = ideal_of<V, SIDE>(k);
+      const V t = A::add(n[k], dk);
+      const V t2 = A::mul(t, t);
+      const V t6 = A::mul(A::mul(t2, t2), t2);
+      const V u = A::fma(n[k], n[k], n[k]);
+      const V u3 = A::mul(A::mul(u, u), u);
+      const V den = A::fma(A::c(-2000.), u3, t6);
+      m[k] = A::fma(A::mul(t6, t), A::rcp(den), A::neg(dk));
     }
-    const float2 tot = add2(add2(add2(add2(m[0], m[1]), m[2]), m[3]), m[4]);
-    r = make_float2(do_map.x ? fast_rcp(tot.x) : 1.f, do_map.y ? fast_rcp(tot.y) : 1.f);
+    r = A::sel(do_map, A::rcp(sum5(m)), r);
 #pragma unroll
-    for (int k = 0; k < 5; k++) w[k] = make_float2(do_map.x ? m[k].x : w[k].x, do_map.y ? m[k].y : w[k].y);
+    for (int k = 0; k < 5; k++) n[k] = A::sel(do_map, m[k], n[k]);
   }
-  float2 acc = f2(0.f);
-#pragma unroll
-  for (int k = 0; k < 5; k++) {
-    float2 lin = mul2(lin2<SIDE>(k, 0), d[k]);
-#pragma unroll
-    for (int m = 1; m < 4; m++) lin = fma2(lin2<SIDE>(k, m), d[k + m], lin);
-    acc = fma2(w[k], lin, acc);
-  }
-  return fma2(acc, r, s4);
+  return r;
 }
 
-// Stencil differences and the shared reciprocals rk = 1/(TV_k^2 + 1e-20) of
-// two stencils.
-__device__ __forceinline__ void weno9_rk2(const float2 (&s)[9], float2 (&d)[8], float2 (&rk)[5], bool2 imm_L,
-                                          bool2 imm_R) {
-  using namespace pu_weno9;
+template <class V, int SIDE>
+__device__ __forceinline__ V weno9_edge(const V (&X)[5], const V (&O)[5], V s4, const V (&rk)[5],
+                                        typename Arith<V>::B do_map) {
+  using A = Arith<V>;
+  V n[5];
+  const V r = weno9_neg_weights<V, SIDE>(rk, do_map, n);
+  V acc = A::mul(n[0], A::fma(odd_of<V, SIDE>(), O[0], X[0]));
 #pragma unroll
-  for (int m = 0; m < 8; m++) d[m] = sub2(s[m + 1], s[m]);
-  float2 tv[5];
-#pragma unroll
-  for (int k = 0; k < 5; k++) {
-    const float2 y3 = d[k + 3];
-    const float2 y2 = fma2(f2(float(TV_L[k][3][2])), d[k + 3], d[k + 2]);
-    const float2 y1 = fma2(f2(float(TV_L[k][3][1])), d[k + 3], fma2(f2(float(TV_L[k][2][1])), d[k + 2], d[k + 1]));
-    const float2 y0 = fma2(f2(float(TV_L[k][3][0])), d[k + 3],
-                           fma2(f2(float(TV_L[k][2][0])), d[k + 2], fma2(f2(float(TV_L[k][1][0])), d[k + 1], d[k])));
-    float2 t = mul2(mul2(f2(float(TV_D[k][3])), y3), y3);
-    t = fma2(mul2(f2(float(TV_D[k][2])), y2), y2, t);
-    t = fma2(mul2(f2(float(TV_D[k][1])), y1), y1, t);
-    tv[k] = fma2(mul2(f2(float(TV_D[k][0])), y0), y0, t);
-  }
-  convexify5x2(tv);
-  if (imm_L.x || imm_L.y || imm_R.x || imm_R.y) {
-    const float mx = fmaxf(fmaxf(fmaxf(fmaxf(tv[0].x, tv[1].x), tv[2].x), tv[3].x), tv[4].x);
-    const float my = fmaxf(fmaxf(fmaxf(fmaxf(tv[0].y, tv[1].y), tv[2].y), tv[3].y), tv[4].y);
-    if (imm_L.x) tv[4].x = mx;
-    if (imm_L.y) tv[4].y = my;
-    if (imm_R.x) tv[0].x = mx;
-    if (imm_R.y) tv[0].y = my;
-  }
-#pragma unroll
-  for (int k = 0; k < 5; k++) rk[k] = rcp2(fma2(tv[k], tv[k], f2(1.e-20f)));
+  for (int k = 1; k < 5; k++) acc = A::fma(n[k], A::fma(odd_of<V, SIDE>(), O[k], X[k]), acc);
+  return A::fma(acc, A::mul(r, A::c(pu_weno9::DF_OUT)), s4);
 }
 
-__device__ __forceinline__ void weno9_edges2(const float2 (&s)[9], float2 &qL, float2 &qR, bool2 do_map, bool2 imm_L,
-                                             bool2 imm_R) {
-  float2 d[8], rk[5];
-  weno9_rk2(s, d, rk, imm_L, imm_R);
-  qL = weno9_edge2<0>(d, s[4], rk, do_map);
-  qR = weno9_edge2<1>(d, s[4], rk, do_map);
+// Both edges of one stencil (R float or double) or of two (float2).
+template <class V>
+__device__ __forceinline__ void weno9_edges(const V (&s)[9], V &qL, V &qR, typename Arith<V>::B do_map,
+                                            typename Arith<V>::B imm_L, typename Arith<V>::B imm_R) {
+  V X[5], O[5], tv[5], rk[5];
+  weno9_windows(s, X, O, tv);
+  weno9_rk(tv, imm_L, imm_R, rk);
+  qL = weno9_edge<V, 0>(X, O, s[4], rk, do_map);
+  qR = weno9_edge<V, 1>(X, O, s[4], rk, do_map);
 }
 
 // The right edge of stencil x and the left edge of stencil y, each
-// bit-identical to that edge from weno9_edges2: the one edge a tile needs
+// bit-identical to that edge from weno9_edges: the one edge a tile needs
 // from each of the two halo cells that close a row of faces.
 __device__ __forceinline__ float2 weno9_outer_edges2(const float2 (&s)[9], bool2 do_map, bool2 imm_L, bool2 imm_R) {
-  float2 d[8], rk[5];
-  weno9_rk2(s, d, rk, imm_L, imm_R);
-  return weno9_edge2<2>(d, s[4], rk, do_map);
+  float2 X[5], O[5], tv[5], rk[5];
+  weno9_windows(s, X, O, tv);
+  weno9_rk(tv, imm_L, imm_R, rk);
+  return weno9_edge<float2, 2>(X, O, s[4], rk, do_map);
 }
 
-// Normalised nonlinear weights of the left edge (after map_rs when do_map),
-// the quantity the learned network is trained to reproduce.
+// Normalised nonlinear weights of the left edge after map_rs, the quantity
+// the learned network is trained to reproduce.
 template <class R>
 __device__ __forceinline__ void weno9_left_weights(const R (&s)[9], R (&w)[5]) {
-  using namespace pu_weno9;
-  R d[8];
+  R X[5], O[5], tv[5], rk[5], n[5];
+  weno9_windows(s, X, O, tv);
+  weno9_rk(tv, false, false, rk);
+  const R r = weno9_neg_weights<R, 0>(rk, true, n);
 #pragma unroll
-  for (int m = 0; m < 8; m++) d[m] = s[m + 1] - s[m];
-  R tv[5];
-#pragma unroll
-  for (int k = 0; k < 5; k++) {
-    R y3 = d[k + 3];
-    R y2 = fma(R(TV_L[k][3][2]), d[k + 3], d[k + 2]);
-    R y1 = fma(R(TV_L[k][3][1]), d[k + 3], fma(R(TV_L[k][2][1]), d[k + 2], d[k + 1]));
-    R y0 = fma(R(TV_L[k][3][0]), d[k + 3], fma(R(TV_L[k][2][0]), d[k + 2], fma(R(TV_L[k][1][0]), d[k + 1], d[k])));
-    R t = R(TV_D[k][3]) * y3 * y3;
-    t = fma(R(TV_D[k][2]) * y2, y2, t);
-    t = fma(R(TV_D[k][1]) * y1, y1, t);
-    tv[k] = fma(R(TV_D[k][0]) * y0, y0, t);
-  }
-  convexify5(tv);
-#pragma unroll
-  for (int k = 0; k < 5; k++) w[k] = R(IDEAL_L[k]) * fast_rcp(fma(tv[k], tv[k], R(1.e-20)));
-  convexify5(w);
-#pragma unroll
-  for (int k = 0; k < 5; k++) {
-    const R dk = R(IDEAL_L[k]);
-    R t = w[k] - dk;
-    R t2 = t * t;
-    R t6 = t2 * t2 * t2;
-    R u = fma(-w[k], w[k], w[k]);
-    R u3 = u * u * u;
-    w[k] = fma(t6 * t, fast_rcp(fma(R(2000.), u3, t6)), dk);
-  }
-  convexify5(w);
+  for (int k = 0; k < 5; k++) w[k] = n[k] * r;
 }
 
 // Edge values from given left-edge and right-edge weights (the last step of
