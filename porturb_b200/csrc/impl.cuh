@@ -284,20 +284,19 @@ struct ImplBase {
     return PU_OK;
   }
 
-  // One forward/backward over `batch` samples of (xs, ts): gradient in ml_grad.
-  int ml_fwd_bwd(const float *xs, const float *ts, long ndata, int batch, unsigned long long seed, int sequential) {
-    const int nb = (batch + mlp::TB - 1) / mlp::TB;
+  // One forward/backward over `batch` samples of (xs, ts): the blocks' partial
+  // gradients (nb of them) in ml_partial.
+  int ml_fwd_bwd(const float *xs, const float *ts, long ndata, int batch, unsigned long long seed, int sequential,
+                 int &nb) {
+    nb = (batch + mlp::TB - 1) / mlp::TB;
     int rc = ml_partials(nb);
     if (rc) return rc;
-    PU_CK(cudaFuncSetAttribute(k_mlp_fwd_bwd, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               int(mlp_train_smem_bytes())));
-    k_mlp_fwd_bwd<<<nb, mlp::TB, mlp_train_smem_bytes(), st>>>(ml_wq, xs, ts, ndata, ml_step, seed, batch, sequential,
-                                                               ml_partial);
-    PU_LAUNCHED();
-    k_mlp_reduce<<<(mlp::NPARAM + 1 + 255) / 256, 256, 0, st>>>(ml_partial, nb, ml_grad);
+    k_mlp_fwd_bwd<<<nb, mlp::TB, mlp::SM_FLOATS * sizeof(float), st>>>(ml_wq, xs, ts, ndata, ml_step, seed, batch,
+                                                                       sequential, ml_partial);
     PU_LAUNCHED();
     return PU_OK;
   }
+  static constexpr unsigned ML_UPDATE_BLOCKS = (mlp::NPARAM + 1 + 31) / 32;
 
   int ml_train(int steps, int batch, double lr, unsigned long long seed, pu_learn_stats *out) {
     if (ml_n <= 0) {
@@ -310,21 +309,21 @@ struct ImplBase {
     cudaEventRecord(e0, st);
     float loss0 = 0, loss1 = 0;
     for (int it = 0; it < steps; it++) {
-      int rc = ml_fwd_bwd(ml_xs, ml_ts, ml_n, batch, seed, 0);
+      int nb;
+      int rc = ml_fwd_bwd(ml_xs, ml_ts, ml_n, batch, seed, 0, nb);
       if (rc) return rc;
+      ml_step++;
+      const float b1 = 0.9f, b2 = 0.999f;
+      const float bc1 = float(1.0 - std::pow(0.9, double(ml_step))), bc2 = float(1.0 - std::pow(0.999, double(ml_step)));
+      k_mlp_update<true><<<ML_UPDATE_BLOCKS, 1024, 0, st>>>(ml_partial, nb, ml_grad, ml_theta, ml_m, ml_v, ml_wq,
+                                                           float(lr), b1, b2, 1e-8f, bc1, bc2);
+      PU_LAUNCHED();
       if (it == 0 || it == steps - 1) {
         float L;
         PU_CK(cudaMemcpyAsync(&L, ml_grad + mlp::NPARAM, sizeof(float), cudaMemcpyDeviceToHost, st));
         PU_CK(cudaStreamSynchronize(st));
         (it == 0 ? loss0 : loss1) = L / batch;
       }
-      ml_step++;
-      const float b1 = 0.9f, b2 = 0.999f;
-      const float bc1 = float(1.0 - std::pow(0.9, double(ml_step))), bc2 = float(1.0 - std::pow(0.999, double(ml_step)));
-      k_adam<<<(mlp::NPARAM + 255) / 256, 256, 0, st>>>(ml_theta, ml_m, ml_v, ml_grad, float(lr), b1, b2, 1e-8f, bc1, bc2);
-      PU_LAUNCHED();
-      k_mlp_prepare<<<(mlp::NPARAM + 255) / 256, 256, 0, st>>>(ml_theta, ml_wq);
-      PU_LAUNCHED();
     }
     cudaEventRecord(e1, st);
     PU_CK(cudaEventSynchronize(e1));
@@ -381,7 +380,19 @@ struct ImplBase {
     float *dx = static_cast<float *>(p), *dt = dx + n * 9;
     cudaMemcpyAsync(dx, x, size_t(n) * 9 * sizeof(float), cudaMemcpyHostToDevice, st);
     cudaMemcpyAsync(dt, t, size_t(n) * 5 * sizeof(float), cudaMemcpyHostToDevice, st);
-    int rc = ml_fwd_bwd(dx, dt, n, int(n), 0, 1);
+    int nb;
+    int rc = ml_fwd_bwd(dx, dt, n, int(n), 0, 1, nb);
+    if (!rc) {
+      k_mlp_update<false><<<ML_UPDATE_BLOCKS, 1024, 0, st>>>(ml_partial, nb, ml_grad, nullptr, nullptr, nullptr, nullptr,
+                                                             0.f, 0.f, 0.f, 0.f, 1.f, 1.f);
+      const cudaError_t e = cudaGetLastError();
+      if (e != cudaSuccess) {
+        set_error(std::string("kernel launch: ") + cudaGetErrorString(e));
+        rc = PU_ERR_CUDA;
+      } else {
+        launches++;
+      }
+    }
     float h[mlp::NPARAM + 1];
     if (!rc && cudaMemcpyAsync(h, ml_grad, sizeof(h), cudaMemcpyDeviceToHost, st) == cudaSuccess &&
         cudaStreamSynchronize(st) == cudaSuccess) {

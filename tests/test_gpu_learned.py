@@ -46,6 +46,23 @@ def test_gradient_matches_numpy_oracle(gpu_lib):
         assert r < 3e-3, (name, r)
 
 
+@pytest.mark.parametrize("n", [1, 31, 127, 128, 129, 511, 4101])
+def test_gradient_at_the_edges_of_a_block(gpu_lib, n):
+    """Batches around the training block's 128 samples and its warps' 32, and
+    over several rounds of the update kernel's 32 rows.  Bound: an activation
+    whose sum lies within FP32 rounding of a bfloat16 boundary rounds to the
+    neighbour (2^-8 of it, one of 32 in its layer) in the kernel and not in
+    the FP64 oracle."""
+    g = _handle()
+    theta = (mo.init_params(3) * 1.2).astype(np.float32)
+    g.learned_set_weights(theta)
+    x, t = _random_batch(n, seed=n)
+    grad, loss = g.learned_gradient(x, t)
+    loss_o, grad_o = mo.loss_and_grad(theta.astype(np.float64), x, t)
+    assert abs(loss - loss_o) < 1e-3 * abs(loss_o)
+    assert np.linalg.norm(grad - grad_o) < 5e-3 * np.linalg.norm(grad_o)
+
+
 @pytest.mark.parametrize("use_mma", [False, True])
 def test_eval_matches_numpy_oracle(gpu_lib, use_mma):
     g = _handle()
