@@ -53,6 +53,8 @@ namespace pu {
 #ifndef PU_XY_MIN_BLOCKS
 #define PU_XY_MIN_BLOCKS 4
 #endif
+// (FP64: 512 threads per SM, i.e. at most 128 registers; uncapped the
+// 16x16 tile takes 130-136 and one block per SM.)
 // Minimum resident blocks per SM requested for the plain z march: 4 blocks
 // of 128 threads (at most 128 registers) measured 0.4 % faster than no cap.
 #ifndef PU_Z_MIN_BLOCKS
@@ -67,6 +69,10 @@ namespace pu {
 // (256 threads: 4 blocks cap it at 64 registers, as the x/y kernel).
 #ifndef PU_ZT_MIN_BLOCKS
 #define PU_ZT_MIN_BLOCKS 4
+#endif
+// The same in FP64: 2 blocks (128 registers; 56 KB of shared memory each).
+#ifndef PU_ZT_MIN_BLOCKS_F64
+#define PU_ZT_MIN_BLOCKS_F64 2
 #endif
 #ifndef PU_LEARNED_Z_MIN_BLOCKS
 #define PU_LEARNED_Z_MIN_BLOCKS 3
@@ -490,6 +496,51 @@ __device__ __forceinline__ void recon_outer_pair(int f, int line, Load load, Sto
   store_outer(f, line, q.x, q.y);
 }
 
+// The same lines in FP64 (weno_all): one stencil at a time, a thread walking
+// the fields of one position where there is a thread per position, and the
+// one edge needed from each of the two halo cells that close a line.
+template <int NT, int F, int LINES, int W, bool POS_MAJOR, class Mask, class Vals, class Store>
+__device__ __forceinline__ void recon_f64_inner(Mask mask, Vals vals, Store store) {
+  constexpr int P = LINES * W;
+  for (int p = threadIdx.x; p < P; p += NT) {
+    const int line = POS_MAJOR ? p % LINES : p / W, pos = (POS_MAJOR ? p / LINES : p % W) + 1;
+    unsigned im;
+    bool ax;
+    mask(line, pos, im, ax);
+#pragma unroll 1
+    for (int f = 0; f < F; f++) {
+      double s[9], qL, qR;
+      vals(f, line, pos, s, im);
+      weno9_edges(s, qL, qR, !ax, ((im >> 3) & 1u) != 0, ((im >> 5) & 1u) != 0);
+      store(f, line, pos, qL, qR);
+    }
+  }
+}
+
+template <int W, class Load, class StoreOuter>
+__device__ __forceinline__ void recon_f64_outer_pair(int f, int line, Load load, StoreOuter store_outer) {
+  double s[9];
+  unsigned im;
+  bool ax;
+  load(f, line, 0, s, im, ax);
+  const double qR0 = weno9_one_edge<false>(s, !ax, ((im >> 3) & 1u) != 0, ((im >> 5) & 1u) != 0);
+  load(f, line, W + 1, s, im, ax);
+  const double qL1 = weno9_one_edge<true>(s, !ax, ((im >> 3) & 1u) != 0, ((im >> 5) & 1u) != 0);
+  store_outer(f, line, qR0, qL1);
+}
+
+// Lines of the stencil type: packed pairs in FP32, one by one in FP64.
+template <class R, int NT, int F, int LINES, int W, bool POS_MAJOR, class Mask, class Vals, class Store>
+__device__ __forceinline__ void recon_inner(Mask mask, Vals vals, Store store) {
+  if constexpr (std::is_same<R, float>::value) recon_packed_inner<NT, F, LINES, W, POS_MAJOR>(mask, vals, store);
+  else recon_f64_inner<NT, F, LINES, W, POS_MAJOR>(mask, vals, store);
+}
+template <class R, int W, class Load, class StoreOuter>
+__device__ __forceinline__ void recon_outer(int f, int line, Load load, StoreOuter store_outer) {
+  if constexpr (std::is_same<R, float>::value) recon_outer_pair<W>(f, line, load, store_outer);
+  else recon_f64_outer_pair<W>(f, line, load, store_outer);
+}
+
 // x/y fluxes and their divergence for one (x,y) tile of one level.
 // LEARNED (FP32, weno_all only): edges from the network's weights, with the
 // plain limiter as the fallback.
@@ -499,7 +550,7 @@ __device__ __forceinline__ void recon_outer_pair(int f, int line, Load load, Sto
 // a precursor edge, partial tiles and halo boxes that would straddle the
 // domain's edge are loaded by the threads.
 template <class R, int NTR, int TX, int TY, bool IMM, bool LEARNED = false, bool DECOMP = false, bool TMA = false>
-__global__ void __launch_bounds__(TX *TY, LEARNED ? PU_LEARNED_XY_MIN_BLOCKS : (sizeof(R) == 4 ? PU_XY_MIN_BLOCKS : 1)) k_xy(const Grid<R> G, const R *__restrict__ sin, R *__restrict__ txy, const __grid_constant__ XyMaps maps) {
+__global__ void __launch_bounds__(TX *TY, LEARNED ? PU_LEARNED_XY_MIN_BLOCKS : (sizeof(R) == 4 ? PU_XY_MIN_BLOCKS : 512 / (TX * TY))) k_xy(const Grid<R> G, const R *__restrict__ sin, R *__restrict__ txy, const __grid_constant__ XyMaps maps) {
   using Sh = XYShape<R, NTR, TX, TY, IMM, LEARNED>;
   constexpr int F = Sh::F, S = Sh::S, NT = Sh::NT, HX = Sh::HX, HY = Sh::HY, EN = Sh::EN, FN = Sh::FN;
   static_assert(!TMA || (Sh::TMA_FITS && !DECOMP && !IMM), "TMA staging: 16x16 FP32 tiles, plain domains");
@@ -697,23 +748,23 @@ __global__ void __launch_bounds__(TX *TY, LEARNED ? PU_LEARNED_XY_MIN_BLOCKS : (
   };
   int n_fb = 0;
   bool packed = false;
-  if constexpr (std::is_same<R, float>::value && PU_PACKED_LIMITER && !LEARNED) {
+  if constexpr ((!std::is_same<R, float>::value || PU_PACKED_LIMITER) && !LEARNED) {
     packed = G.weno_all != 0;
     if (packed) {
-      recon_packed_inner<NT, F, TY, TX, false>(mask_xc, vals_xc, store_xc);
+      recon_inner<R, NT, F, TY, TX, false>(mask_xc, vals_xc, store_xc);
       // Halo pairs of the x lines, and already those of the y lines (kept in
       // YO until the y phase), so that every thread takes one pair here and
       // the y phase is the inner rounds alone.
       const int nxo = F * TY, nyo = sim2d ? 0 : F * TX;
       for (int p = tid; p < nxo + nyo; p += NT) {
         if (p < nxo) {
-          recon_outer_pair<TX>(p / TY, p % TY, load_xc, [&](int f, int r, R qR0, R qL1) {
+          recon_outer<R, TX>(p / TY, p % TY, load_xc, [&](int f, int r, R qR0, R qL1) {
             ER[f * EN + r * (TX + 2)] = qR0;
             EL[f * EN + r * (TX + 2) + TX + 1] = qL1;
           });
         } else {
           const int q = p - nxo;
-          recon_outer_pair<TY>(q / TX, q % TX, load_yc, [&](int f, int cc, R qR0, R qL1) {
+          recon_outer<R, TY>(q / TX, q % TX, load_yc, [&](int f, int cc, R qR0, R qL1) {
             YO[f * TX + cc] = qR0;
             YO[(F + f) * TX + cc] = qL1;
           });
@@ -784,16 +835,14 @@ __global__ void __launch_bounds__(TX *TY, LEARNED ? PU_LEARNED_XY_MIN_BLOCKS : (
       __syncthreads();   // step 4 has read the flux buffer that holds the queue
       n_fb += recon_learned<NT>(G, sW, queue, qn + 1, F * Sh::EYN, load_y, store_y);
     } else if (packed) {
-      if constexpr (std::is_same<R, float>::value) {
-        recon_packed_inner<NT, F, TX, TY, true>(mask_yc, vals_yc, [&](int f, int cc, int rr, R qL, R qR) {
-          EL[f * EN + rr * TX + cc] = qL;
-          ER[f * EN + rr * TX + cc] = qR;
-        });
-        for (int p = tid; p < F * TX; p += NT) {   // the halo-cell edges taken in the x phase
-          const int f = p / TX, cc = p % TX;
-          ER[f * EN + cc] = YO[p];
-          EL[f * EN + (TY + 1) * TX + cc] = YO[F * TX + p];
-        }
+      recon_inner<R, NT, F, TX, TY, true>(mask_yc, vals_yc, [&](int f, int cc, int rr, R qL, R qR) {
+        EL[f * EN + rr * TX + cc] = qL;
+        ER[f * EN + rr * TX + cc] = qR;
+      });
+      for (int p = tid; p < F * TX; p += NT) {   // the halo-cell edges taken in the x phase
+        const int f = p / TX, cc = p % TX;
+        ER[f * EN + cc] = YO[p];
+        EL[f * EN + (TY + 1) * TX + cc] = YO[F * TX + p];
       }
     } else {
       for (int it = tid; it < F * Sh::EYN; it += NT) {
@@ -1174,25 +1223,25 @@ __global__ void __launch_bounds__(TX *TY, LEARNED ? PU_LEARNED_Z_MIN_BLOCKS : (s
 // step's initial state and the x/y tendency of levels k0 .. k0+TZ-1
 // ([S][TZ][TX] each) -- land in buffers of their own, copied while the block
 // reconstructs.  Two mbarriers complete the copies.
-template <int NTR, int TX, int TZ, bool IMM = false>
+template <class R, int NTR, int TX, int TZ, bool IMM = false>
 struct ZTShape {
   static constexpr int F = 6 + NTR, S = 5 + NTR, NT = TX * TZ, HZ = TZ + 10;
   static constexpr int EN = (TZ + 2) * TX;
   static constexpr size_t al(size_t b) { return (b + 127) / 128 * 128; }
   // Immersed domains add one flag byte per level and column (bit 0 immersed,
   // bit 1 an immersed cell within 10).
-  static constexpr size_t base_bytes = sizeof(float) * (size_t(F) * HZ * TX + 2 * size_t(F) * EN) +
+  static constexpr size_t base_bytes = sizeof(R) * (size_t(F) * HZ * TX + 2 * size_t(F) * EN) +
                                        (IMM ? (size_t(HZ) * TX + 15) / 16 * 16 : 0);
   static constexpr size_t bytes = base_bytes;
   // The TMA instantiation rounds the start of its dynamic shared memory up to
   // 128 bytes (the alignment of the TMA destinations): PAD bytes more.
   static constexpr size_t PAD = 128;
   // TMA staging (byte offsets from the start of shared memory).
-  static constexpr size_t el_off = sizeof(float) * size_t(F) * HZ * TX;
+  static constexpr size_t el_off = sizeof(R) * size_t(F) * HZ * TX;
   static constexpr size_t raw_off = al(el_off);
-  static constexpr size_t raw_bytes = sizeof(float) * size_t(S) * HZ * TX;
-  static constexpr size_t cell_bytes = sizeof(float) * size_t(S) * TZ * TX;
-  static_assert(raw_off + raw_bytes <= el_off + sizeof(float) * 2 * size_t(F) * EN, "raw tile exceeds the edge buffers");
+  static constexpr size_t raw_bytes = sizeof(R) * size_t(S) * HZ * TX;
+  static constexpr size_t cell_bytes = sizeof(R) * size_t(S) * TZ * TX;
+  static_assert(raw_off + raw_bytes <= el_off + sizeof(R) * 2 * size_t(F) * EN, "raw tile exceeds the edge buffers");
   static constexpr size_t cells_off = al(base_bytes);
   static constexpr size_t bar_off = cells_off + 3 * cell_bytes;
   static constexpr size_t tma_bytes_prefetch = bar_off + 16;
@@ -1217,9 +1266,14 @@ struct ZtMaps {
 // of the TZ inner cells of each column come from the packed limiter two
 // stencils per thread, the two cells that close a column (k0-1: right edge,
 // k0+TZ: left edge) from its one-edge form; then each thread takes the
-// Riemann fluxes through the two faces of its cell and finalises it.  FP32
-// with weno_all (IMM: domains with immersed cells, whose level flags go to
-// shared memory with the fields); every other form keeps the march.
+// Riemann fluxes through the two faces of its cell and finalises it.  With
+// weno_all (IMM: domains with immersed cells, whose level flags go to shared
+// memory with the fields); every other form keeps the march.
+// FP64 takes the tile as well, one stencil at a time (56 KB of shared memory,
+// two blocks per SM): with the three-division limiter the 256x4x128 bubble
+// runs ten steps in 2.88 ms against 9.67 ms for the march (64 blocks there,
+// fewer than the SMs) and the 128x128x96 boundary layer two steps in 5.78
+// against 10.5 ms; the FP64 pipe is 72 % busy here and 82 % in k_xy.
 //
 // TMA: the raw tile and the finalisation's cell inputs come from TMA copies
 // (maps: tensor maps of sin, sn and txy); rows the halo box does not hold
@@ -1227,13 +1281,12 @@ struct ZtMaps {
 // fit, the cell inputs are read per thread as without it.  Columns beyond
 // the domain read zero there instead of the last column; their results are
 // discarded either way.
-template <int NTR, int TX, int TZ, bool IMM, bool TMA = false>
-__global__ void __launch_bounds__(TX *TZ, PU_ZT_MIN_BLOCKS) k_zt(const Grid<float> G, const float *__restrict__ sin,
-                                                               const float *sn, float *sout,
-                                                               const float *__restrict__ txy, float a_n, float a_dt,
-                                                               int n_enforce, const __grid_constant__ ZtMaps maps) {
-  using R = float;
-  using Sh = ZTShape<NTR, TX, TZ, IMM>;
+template <class R, int NTR, int TX, int TZ, bool IMM, bool TMA = false>
+__global__ void __launch_bounds__(TX *TZ, sizeof(R) == 4 ? PU_ZT_MIN_BLOCKS : PU_ZT_MIN_BLOCKS_F64)
+    k_zt(const Grid<R> G, const R *__restrict__ sin, const R *sn, R *sout, const R *__restrict__ txy, R a_n, R a_dt,
+         int n_enforce, const __grid_constant__ ZtMaps maps) {
+  static_assert(!TMA || sizeof(R) == 4, "TMA staging: FP32");
+  using Sh = ZTShape<R, NTR, TX, TZ, IMM>;
   constexpr int F = Sh::F, S = Sh::S, NT = Sh::NT, HZ = Sh::HZ;
   extern __shared__ __align__(16) unsigned char smem_zt[];
   unsigned char *smem_raw = TMA ? smem_zt + ((128u - (tma::saddr(smem_zt) & 127u)) & 127u) : smem_zt;
@@ -1353,12 +1406,12 @@ __global__ void __launch_bounds__(TX *TZ, PU_ZT_MIN_BLOCKS) k_zt(const Grid<floa
     mask(c, q, imm, any10);
     vals(f, c, q, s, imm);
   };
-  recon_packed_inner<NT, F, TX, TZ, true>(mask, vals, [&](int f, int c, int q, R qL, R qR) {
+  recon_inner<R, NT, F, TX, TZ, true>(mask, vals, [&](int f, int c, int q, R qL, R qR) {
     EL[(f * (TZ + 2) + q) * TX + c] = qL;
     ER[(f * (TZ + 2) + q) * TX + c] = qR;
   });
   for (int pr = tid; pr < F * TX; pr += NT)
-    recon_outer_pair<TZ>(pr / TX, pr % TX, load, [&](int f, int c, R qR0, R qL1) {
+    recon_outer<R, TZ>(pr / TX, pr % TX, load, [&](int f, int c, R qR0, R qL1) {
       ER[(f * (TZ + 2)) * TX + c] = qR0;
       EL[(f * (TZ + 2) + TZ + 1) * TX + c] = qL1;
     });
@@ -1409,7 +1462,7 @@ __global__ void __launch_bounds__(TX *TZ, PU_ZT_MIN_BLOCKS) k_zt(const Grid<floa
   for (int s2 = 0; s2 < S; s2++) {
     qin[s2] = pref ? QIN[s2 * TZ * TX + cq] : sin[s2 * G.N + idx];
     tx[s2] = pref ? TXY[s2 * TZ * TX + cq] : txy[s2 * G.N + idx];
-    dF[s2] = __fsub_rn(Ft[s2], Fb[s2]);   // not fused with the flux products: the march's bits
+    dF[s2] = Arith<R>::sub(Ft[s2], Fb[s2]);   // not fused with the flux products: the march's bits
   }
   finish_cell<R, NTR, IMM>(
       G, qin, tx, [&](int s2) { return pref ? SN[s2 * TZ * TX + cq] : sn[s2 * G.N + idx]; }, dF, sn != nullptr,

@@ -752,15 +752,15 @@ struct Impl : ImplBase {
                                int(ZShape<R, NTR, ZTX, ZTY>::bytes)));
     PU_CK(cudaFuncSetAttribute(k_z<R, NTR, ZTX, ZTY, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                int(ZShape<R, NTR, ZTX, ZTY>::bytes)));
+    PU_CK(cudaFuncSetAttribute(k_zt<R, NTR, ZT_X, ZT_Z, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               int(ZTShape<R, NTR, ZT_X, ZT_Z, false>::bytes)));
+    PU_CK(cudaFuncSetAttribute(k_zt<R, NTR, ZT_X, ZT_Z, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               int(ZTShape<R, NTR, ZT_X, ZT_Z, true>::bytes)));
     if constexpr (std::is_same<R, float>::value) {
-      PU_CK(cudaFuncSetAttribute(k_zt<NTR, ZT_X, ZT_Z, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 int(ZTShape<NTR, ZT_X, ZT_Z, false>::bytes)));
-      PU_CK(cudaFuncSetAttribute(k_zt<NTR, ZT_X, ZT_Z, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 int(ZTShape<NTR, ZT_X, ZT_Z, true>::bytes)));
-      PU_CK(cudaFuncSetAttribute(k_zt<NTR, ZT_X, ZT_Z, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 int(ZTShape<NTR, ZT_X, ZT_Z, false>::tma_bytes)));
-      PU_CK(cudaFuncSetAttribute(k_zt<NTR, ZT_X, ZT_Z, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 int(ZTShape<NTR, ZT_X, ZT_Z, true>::tma_bytes)));
+      PU_CK(cudaFuncSetAttribute(k_zt<R, NTR, ZT_X, ZT_Z, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 int(ZTShape<R, NTR, ZT_X, ZT_Z, false>::tma_bytes)));
+      PU_CK(cudaFuncSetAttribute(k_zt<R, NTR, ZT_X, ZT_Z, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 int(ZTShape<R, NTR, ZT_X, ZT_Z, true>::tma_bytes)));
       if constexpr (XYShape<R, NTR, XTX_BIG, XTY_BIG, false>::TMA_FITS)
         PU_CK(cudaFuncSetAttribute(k_xy<R, NTR, XTX_BIG, XTY_BIG, false, false, false, true>,
                                    cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1039,11 +1039,11 @@ struct Impl : ImplBase {
   // every level for a decomposed tile or when the config asks for it.
   int imm_levels() const { return (dc.on || cfg.imm_all_levels || !has_imm) ? cfg.nz : imm_kc; }
 
-  // The tiled z kernel (k_zt) takes the plain FP32 limiter with weno_all,
-  // unless a z chunk was asked for (the march, which gives the same bits).  Its grid has one y row per block
-  // row, so ny is held to the grid's y limit.
+  // The tiled z kernel (k_zt) takes the plain limiter with weno_all, unless a
+  // z chunk was asked for (the march; in FP32 it gives the same bits).  Its
+  // grid has one y row per block row, so ny is held to the grid's y limit.
   bool z_tiled(bool learned) const {
-    return std::is_same<R, float>::value && cfg.weno_all && !learned && cfg.z_chunk <= 0 && cfg.ny <= 65535;
+    return cfg.weno_all && !learned && cfg.z_chunk <= 0 && cfg.ny <= 65535;
   }
 
   // Learned weights replace the nonlinear limiter where it runs on every
@@ -1097,50 +1097,45 @@ struct Impl : ImplBase {
     return PU_OK;
   }
 
-  // The tiled z kernel (FP32, z_tiled) on z chunks [c0, c1) of ZT_Z levels:
-  // chunks below ci take the immersed kernel.  Chunk c reads levels
-  // 32c-5 .. 32c+36, so it is plain once 32c-5 reaches the first level no
-  // flag holds; a periodic z wraps flagged levels into the top chunk, so every
-  // chunk stays immersed there.  The maps of this stage input (s[b]); the
-  // cell maps of sn and txy are the same for every b.
+  // The tiled z kernel on z chunks [c0, c1) of ZT_Z levels; FP32 through TMA
+  // where the stage input is s[b] (the cell maps of sn and txy are the same
+  // for every b).
+  template <bool IMM>
+  int zt_launch(const Grid<R> &G, const R *sin, const R *sn, R *sout, R a_n, R a_dt, int n_enforce, int b, int c0,
+                int c1) {
+    using Zs = ZTShape<R, NTR, ZT_X, ZT_Z, IMM>;
+    if (c1 <= c0) return PU_OK;
+    const R *t = static_cast<const R *>(txy);
+    Grid<R> Gc = G;
+    Gc.c_first = c0;
+    const dim3 g(blocks(cfg.nx, ZT_X), unsigned(cfg.ny), unsigned(c1 - c0));
+    bool staged = false;
+    if constexpr (std::is_same<R, float>::value) {
+      if (zt_tma && static_cast<const void *>(sin) == s[b]) {
+        k_zt<R, NTR, ZT_X, ZT_Z, IMM, true><<<g, ZT_X * ZT_Z, Zs::tma_bytes, st>>>(Gc, sin, sn, sout, t, a_n, a_dt,
+                                                                                 n_enforce, zt_maps[b]);
+        staged = true;
+      }
+    }
+    if (!staged)
+      k_zt<R, NTR, ZT_X, ZT_Z, IMM><<<g, ZT_X * ZT_Z, Zs::bytes, st>>>(Gc, sin, sn, sout, t, a_n, a_dt, n_enforce,
+                                                                     zt_maps[b]);
+    PU_LAUNCHED();
+    return PU_OK;
+  }
+
+  // The tiled z kernel (z_tiled) on z chunks [c0, c1): chunks below ci take
+  // the immersed kernel.  Chunk c reads levels 32c-5 .. 32c+36, so it is plain
+  // once 32c-5 reaches the first level no flag holds; a periodic z wraps
+  // flagged levels into the top chunk, so every chunk stays immersed there.
   template <bool IMM>
   int zt_chunks(const Grid<R> &G, const R *sin, const R *sn, R *sout, R a_n, R a_dt, int n_enforce, int b, int c0,
                 int c1) {
-    if constexpr (std::is_same<R, float>::value) {
-      using Zs = ZTShape<NTR, ZT_X, ZT_Z, IMM>;
-      using Zp = ZTShape<NTR, ZT_X, ZT_Z, false>;
-      R *t = static_cast<R *>(txy);
-      const int nch = int(blocks(cfg.nz, ZT_Z));
-      const int ci0 = !IMM ? 0 : (cfg.bc_z == PU_BC_WALL ? std::min(nch, (imm_levels() + 5 + ZT_Z - 1) / ZT_Z) : nch);
-      const int ci = std::min(std::max(ci0, c0), c1);
-      const bool tma = zt_tma && static_cast<const void *>(sin) == s[b];
-      const unsigned bx = blocks(cfg.nx, ZT_X), by = unsigned(cfg.ny);
-      if (ci > c0) {
-        Grid<R> Gi = G;
-        Gi.c_first = c0;
-        const dim3 gt(bx, by, ci - c0);
-        if (tma)
-          k_zt<NTR, ZT_X, ZT_Z, IMM, true><<<gt, ZT_X * ZT_Z, Zs::tma_bytes, st>>>(Gi, sin, sn, sout, t, a_n, a_dt,
-                                                                                 n_enforce, zt_maps[b]);
-        else
-          k_zt<NTR, ZT_X, ZT_Z, IMM><<<gt, ZT_X * ZT_Z, Zs::bytes, st>>>(Gi, sin, sn, sout, t, a_n, a_dt, n_enforce,
-                                                                          zt_maps[b]);
-        PU_LAUNCHED();
-      }
-      if (ci < c1) {
-        Grid<R> Gp = G;
-        Gp.c_first = ci;
-        const dim3 gt(bx, by, c1 - ci);
-        if (tma)
-          k_zt<NTR, ZT_X, ZT_Z, false, true><<<gt, ZT_X * ZT_Z, Zp::tma_bytes, st>>>(Gp, sin, sn, sout, t, a_n, a_dt,
-                                                                                    n_enforce, zt_maps[b]);
-        else
-          k_zt<NTR, ZT_X, ZT_Z, false><<<gt, ZT_X * ZT_Z, Zp::bytes, st>>>(Gp, sin, sn, sout, t, a_n, a_dt,
-                                                                            n_enforce, zt_maps[b]);
-        PU_LAUNCHED();
-      }
-    }
-    return PU_OK;
+    const int nch = int(blocks(cfg.nz, ZT_Z));
+    const int ci0 = !IMM ? 0 : (cfg.bc_z == PU_BC_WALL ? std::min(nch, (imm_levels() + 5 + ZT_Z - 1) / ZT_Z) : nch);
+    const int ci = std::min(std::max(ci0, c0), c1);
+    PU_TRY((zt_launch<IMM>(G, sin, sn, sout, a_n, a_dt, n_enforce, b, c0, ci)));
+    return zt_launch<false>(G, sin, sn, sout, a_n, a_dt, n_enforce, b, ci, c1);
   }
 
   // One SSPRK3 stage: the x/y kernel (DEC: a decomposed tile reading its
@@ -1178,17 +1173,10 @@ struct Impl : ImplBase {
     const int kc = cfg.z_chunk > 0 ? cfg.z_chunk : (cfg.nz < 16 ? cfg.nz : 16);
     dim3 gz(blocks(cfg.nx, ZTX), blocks(cfg.ny, ZTY), blocks(cfg.nz, kc));
     cudaEvent_t e1 = prof_begin();
-    if constexpr (std::is_same<R, float>::value) {
-      if (z_tiled(L)) {
-        // z chunks [0, ci) take the immersed kernel: chunk c reads levels
-        // 32c-5 .. 32c+36, so it is plain once 32c-5 reaches the first level
-        // no flag holds.  A periodic z wraps flagged levels into the top
-        // chunk: every chunk stays immersed there.  The maps of this stage
-        // input (s[b]); the cell maps of sn and txy are the same for every b.
-        PU_TRY((zt_chunks<IMM>(G, sin, sn, sout, a_n, a_dt, n_enforce, b, 0, int(blocks(cfg.nz, ZT_Z)))));
-        prof_end(1, e1);
-        return PU_OK;
-      }
+    if (z_tiled(L)) {
+      PU_TRY((zt_chunks<IMM>(G, sin, sn, sout, a_n, a_dt, n_enforce, b, 0, int(blocks(cfg.nz, ZT_Z)))));
+      prof_end(1, e1);
+      return PU_OK;
     }
     // The learned z march needs full warps: every block's columns inside the domain.
     if (L && cfg.nx % ZTX == 0 && cfg.ny % ZTY == 0)

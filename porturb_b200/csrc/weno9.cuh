@@ -75,21 +75,14 @@ struct Arith<float> {
 };
 
 template <>
-struct Arith<double> {
+struct Arith<double> {   // the windows; the rest of the FP64 limiter is below
   using V = double;
   using B = bool;
   static __device__ __forceinline__ V c(double a) { return a; }
-  static __device__ __forceinline__ V c2(double, double b) { return b; }
   static __device__ __forceinline__ V add(V a, V b) { return __dadd_rn(a, b); }
   static __device__ __forceinline__ V sub(V a, V b) { return __dsub_rn(a, b); }
   static __device__ __forceinline__ V mul(V a, V b) { return __dmul_rn(a, b); }
   static __device__ __forceinline__ V fma(V a, V b, V x) { return ::fma(a, b, x); }
-  static __device__ __forceinline__ V rcp(V a) { return fast_rcp(a); }
-  static __device__ __forceinline__ V neg(V a) { return -a; }
-  static __device__ __forceinline__ V max(V a, V b) { return fmax(a, b); }
-  static __device__ __forceinline__ B gt(V a, double b) { return a > b; }
-  static __device__ __forceinline__ V sel(B q, V a, V b) { return q ? a : b; }
-  static __device__ __forceinline__ bool any(B q) { return q; }
 };
 
 template <>
@@ -248,6 +241,119 @@ __device__ __forceinline__ void weno9_edges(const V (&s)[9], V &qL, V &qR, typen
   weno9_rk(tv, imm_L, imm_R, rk);
   qL = weno9_edge<V, 0>(X, O, s[4], rk, do_map);
   qR = weno9_edge<V, 1>(X, O, s[4], rk, do_map);
+}
+
+// ---------------------------------------------------------------------------
+// FP64.  A division costs about ten FP64 operations, and the form above takes
+// twenty per stencil; here the range of FP64 lets products stand in for the
+// reciprocals of each group of five,
+//   1/b_k : 1/b_j  =  prod_{i != k} b_i : prod_{i != j} b_i,
+// (b_k = TV_k^2 + 1e-20 in [1e-20, ~1]; the map_rs denominators in [2e-13, 32];
+// products of four stay far inside the range), and the two edges share one
+// division where both need one: three divisions per stencil (both edges), two
+// for one edge.
+// ---------------------------------------------------------------------------
+// Every operation is rounded by itself here too (Arith<double>), so that all
+// instantiations of the stencil kernels give a stencil the same bits.
+// o[k] = product of the other four.
+__device__ __forceinline__ void other_products(const double (&b)[5], double (&o)[5]) {
+  using A = Arith<double>;
+  const double b01 = A::mul(b[0], b[1]), b34 = A::mul(b[3], b[4]);
+  const double b012 = A::mul(b01, b[2]), b234 = A::mul(b[2], b34);
+  o[0] = A::mul(b[1], b234);
+  o[1] = A::mul(b[0], b234);
+  o[2] = A::mul(b01, b34);
+  o[3] = A::mul(b012, b[4]);
+  o[4] = A::mul(b012, b[3]);
+}
+
+// The weights up to a common factor, from the TVs:
+// P[k] = prod_{i != k} (TV_i^2 + 1e-20) with the normalised TVs.
+__device__ __forceinline__ void weno9_products(double (&tv)[5], bool imm_L, bool imm_R, double (&P)[5]) {
+  using A = Arith<double>;
+  const double tot = sum5(tv);
+  const double r = tot > 4.e-20 / pu_weno9::DF_CA ? 1. / tot : 1.;
+#pragma unroll
+  for (int k = 0; k < 5; k++) tv[k] = A::mul(tv[k], r);
+  if (imm_L || imm_R) {
+    const double mx = fmax(fmax(fmax(fmax(tv[0], tv[1]), tv[2]), tv[3]), tv[4]);
+    if (imm_L) tv[4] = mx;
+    if (imm_R) tv[0] = mx;
+  }
+  double b[5];
+#pragma unroll
+  for (int k = 0; k < 5; k++) b[k] = A::fma(tv[k], tv[k], 1.e-20);
+  other_products(b, P);
+}
+
+// Unnormalised weights ideal_k P_k of one edge.
+template <bool LEFT>
+__device__ __forceinline__ void weno9_raw_weights(const double (&P)[5], double (&w)[5]) {
+  using namespace pu_weno9;
+#pragma unroll
+  for (int k = 0; k < 5; k++) w[k] = Arith<double>::mul(LEFT ? IDEAL_L[k] : IDEAL_R[k], P[k]);
+}
+
+// Weighted sum of the windows' edges (num) and sum of the weights (den) of
+// one edge from its normalised weights, after map_rs when do_map: the mapped
+// weight (d den_k + t_k^7) / den_k times the product of all five den.
+template <bool LEFT>
+__device__ __forceinline__ void weno9_ratio(const double (&X)[5], const double (&O)[5], double (&w)[5], bool do_map,
+                                            double &num, double &den) {
+  using namespace pu_weno9;
+  using A = Arith<double>;
+  den = 1.;
+  if (do_map) {
+    double q[5], o[5];
+#pragma unroll
+    for (int k = 0; k < 5; k++) {
+      const double dk = LEFT ? IDEAL_L[k] : IDEAL_R[k];
+      const double t = A::sub(w[k], dk), t2 = A::mul(t, t), t6 = A::mul(A::mul(t2, t2), t2);
+      const double u = A::fma(-w[k], w[k], w[k]), u3 = A::mul(A::mul(u, u), u);
+      q[k] = A::fma(2000., u3, t6);
+      w[k] = A::fma(dk, q[k], A::mul(t6, t));
+    }
+    other_products(q, o);
+#pragma unroll
+    for (int k = 0; k < 5; k++) w[k] = A::mul(w[k], o[k]);
+    den = sum5(w);
+  }
+  num = A::mul(w[0], A::fma(LEFT ? -DF_SO : DF_SO, O[0], X[0]));
+#pragma unroll
+  for (int k = 1; k < 5; k++) num = A::fma(w[k], A::fma(LEFT ? -DF_SO : DF_SO, O[k], X[k]), num);
+}
+
+template <>
+__device__ __forceinline__ void weno9_edges<double>(const double (&s)[9], double &qL, double &qR, bool do_map,
+                                                    bool imm_L, bool imm_R) {
+  using A = Arith<double>;
+  double X[5], O[5], tv[5], P[5], wl[5], wr[5];
+  weno9_windows(s, X, O, tv);
+  weno9_products(tv, imm_L, imm_R, P);
+  weno9_raw_weights<true>(P, wl);
+  weno9_raw_weights<false>(P, wr);
+  const double sl = sum5(wl), sr = sum5(wr), ri = 1. / A::mul(sl, sr), rl = A::mul(ri, sr), rr = A::mul(ri, sl);
+#pragma unroll
+  for (int k = 0; k < 5; k++) {
+    wl[k] = A::mul(wl[k], rl);
+    wr[k] = A::mul(wr[k], rr);
+  }
+  double nl, dl, nr, dr;
+  weno9_ratio<true>(X, O, wl, do_map, nl, dl);
+  weno9_ratio<false>(X, O, wr, do_map, nr, dr);
+  const double r = pu_weno9::DF_OUT / A::mul(dl, dr);
+  qL = A::fma(nl, A::mul(r, dr), s[4]);
+  qR = A::fma(nr, A::mul(r, dl), s[4]);
+}
+
+// The left or the right edge alone, by the two-edge form: the halo cells that
+// close a row of faces need the bits their own tile gives that edge, and the
+// shared divisions make an edge's last bits depend on both.
+template <bool LEFT>
+__device__ __forceinline__ double weno9_one_edge(const double (&s)[9], bool do_map, bool imm_L, bool imm_R) {
+  double qL, qR;
+  weno9_edges(s, qL, qR, do_map, imm_L, imm_R);
+  return LEFT ? qL : qR;
 }
 
 // The right edge of stencil x and the left edge of stencil y, each

@@ -43,3 +43,18 @@ def test_tiled_z_kernel_gives_the_march_bits(name, gpu_lib):
     assert not np.array_equal(st_t, st0)
     assert np.array_equal(st_t, st_m), np.abs(st_t - st_m).max()
     assert np.array_equal(tr_t, tr_m), np.abs(tr_t - tr_m).max()
+
+
+@pytest.mark.parametrize("name", sorted(CASES))
+def test_tiled_z_kernel_in_fp64(name, gpu_lib):
+    """The FP64 build takes the tile too (weno_all); its arithmetic is the
+    march's up to the contraction of products, so after 4 steps the two agree
+    to FP64 rounding (2^-53, times ~1e4 for the nonlinear weights where a
+    stencil is nearly uniform) of each field's magnitude."""
+    case = CASES[name]()
+    _, _, g = gpu_run(case, "f64", 0, 0.0)
+    dt = 0.9 * g.compute_time_step()
+    st_t, tr_t, _ = gpu_run(case, "f64", 4, dt)
+    st_m, tr_m, _ = gpu_run(case, "f64", 4, dt, z_chunk=16)
+    for a, b in list(zip(st_t, st_m)) + list(zip(tr_t, tr_m)):
+        assert np.abs(a - b).max() <= 1e-12 * max(np.abs(b).max(), 1e-300)
