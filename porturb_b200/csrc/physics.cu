@@ -4,11 +4,13 @@
 //
 // k_les: one 32x8 column tile per block marches up a chunk of levels with a
 // 3-plane ring of the closure's primitive fields (rho_d, u, v, w, theta, K,
-// diffused tracer ratios) and immersed flags in shared memory; each level's
-// x and y face fluxes are computed once per face into shared memory, the
-// z face flux of a column is carried to the next level in registers; the
-// TKE source and the update are fused; the result goes to a separate output
-// (neighbouring blocks still read the input).
+// diffused tracer ratios) and immersed flags in shared memory; the raw fields
+// of the next plane cross by asynchronous copies while a level computes; each
+// thread takes the low x and y faces of its cell (the high x face comes from
+// the next lane, the high y face through shared memory), the z face flux of a
+// column is carried to the next level in registers; the TKE source and the
+// update are fused; the result goes to a separate output (neighbouring blocks
+// still read the input).
 // k_level_partial / k_level_final: deterministic level means (Neumaier-
 // compensated FP64 sums in a fixed order) for the sponge and the
 // geostrophic forcing and the pressure-gradient wind forcings; k_sponge /
@@ -46,7 +48,10 @@ struct Grid {
   double R_d, gamma, C0, grav, rgamma, rgm1;
   int gravity, dns;
   double nu, nu_Pr, total_mult, diss_mult, shear_mult, delta;
-  const double *prop;   // immersed_proportion_halos (nz+2, ny+2, nx+2)
+  double g, rdelta, Rd_C0, C0_Rd;   // gravity (0 when off), 1/delta, R_d/C0, C0/R_d
+  double pc[6];                     // C(gamma, n), n = 1..6: the series of T's update
+  int pser;                         // gamma in [1, 2]: the series may be used
+  const uint8_t *flags;             // F_* of immersed_proportion_halos (nz+2, ny+2, nx+2)
 };
 
 // q[t]: the t-th diffused tracer (resolved on the host, so the kernels index
@@ -64,70 +69,116 @@ __device__ __forceinline__ int wrapi(int i, int n) {
 }
 __device__ __forceinline__ int clampi(int i, int n) { return i < 0 ? 0 : (i >= n ? n - 1 : i); }
 
+// Shared memory of k_les.  The asynchronous copies take every field while two
+// blocks fit an SM (113 KB each); with three diffused tracers those are
+// loaded when the plane is converted.
 template <int ND>
 struct Les {
-  static constexpr int F = 6 + ND, NF = 6 + ND;   // fields in the ring; fluxes per face
+  static constexpr int F = 6 + ND, NF = 5 + ND;   // fields in the ring; fluxes per face
+  static constexpr int PRE = ND < 3 ? F : 6;      // fields copied ahead
   static constexpr size_t ring_bytes = sizeof(double) * 3 * F * HP;
-  static constexpr size_t flux_bytes = sizeof(double) * NF * (TY * (TX + 1) + (TY + 1) * TX);
-  static constexpr size_t bytes = ring_bytes + flux_bytes + 3 * HP;
+  static constexpr size_t flux_bytes = sizeof(double) * NF * ((TY + 1) * TX + TY);
+  static constexpr size_t raw_bytes = sizeof(double) * PRE * HP;
+  static constexpr size_t bytes = ring_bytes + flux_bytes + raw_bytes + 3 * HP;
+  static_assert(2 * (bytes + 1024) <= 228 * 1024, "two blocks per SM");
 };
 
-// One plane p (-1..nz) of the tile with its halo: primitive fields of the
-// closure (les_closure.h:356-365) with the boundary conditions of
-// coupler.h:785-855 and les_closure.h:411-532 applied while loading: periodic
-// x/y (corners wrap in both), precursor x/y copies the edge cell into the
-// halo of interior rows, solid walls copy the edge level with w = 0 and an
-// isentropic density, periodic z wraps.
-template <int ND>
-__device__ void load_plane(const Grid &G, const In &in, int p, int i0, int j0, double *ring, uint8_t *flag) {
-  constexpr int F = Les<ND>::F;
+__device__ __forceinline__ void copy_async8(double *dst, const double *src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst))),
+               "l"(src)
+               : "memory");
+}
+
+// Source cell of tile cell c (halo row c / HX, column c % HX) of plane p
+// (-1..nz) with the boundary conditions of coupler.h:785-855 and
+// les_closure.h:411-532: periodic x/y (corners wrap in both), precursor x/y
+// copies the edge cell into the halo of interior rows, solid walls copy the
+// edge level (zhalo), periodic z wraps.
+__device__ __forceinline__ size_t source_cell(const Grid &G, int c, int p, int i0, int j0, bool &zhalo) {
   const int nx = G.nx, ny = G.ny, nz = G.nz;
+  const int gj = j0 - 1 + c / HX, gi = i0 - 1 + c % HX;
+  const bool inx = gi >= 0 && gi < nx, iny = gj >= 0 && gj < ny;
+  int si = gi, sj = gj;
+  if (!inx && iny) si = G.bc_x == BC_PRECURSOR ? clampi(gi, nx) : wrapi(gi, nx);
+  else if (inx && !iny) sj = G.bc_y == BC_PRECURSOR ? clampi(gj, ny) : wrapi(gj, ny);
+  else if (!inx && !iny) {
+    si = wrapi(gi, nx);
+    sj = wrapi(gj, ny);
+  }
+  int sp = p;
+  zhalo = false;
+  if (p < 0 || p >= nz) {
+    if (G.bc_z == BC_WALL) {
+      sp = p < 0 ? 0 : nz - 1;
+      zhalo = true;
+    } else {
+      sp = wrapi(p, nz);
+    }
+  }
+  return (size_t(sp) * ny + sj) * nx + si;
+}
+
+template <int ND>
+__device__ __forceinline__ const double *field(const In &in, int f) {
+  return f == 0 ? in.rd : f == 1 ? in.u : f == 2 ? in.v : f == 3 ? in.w : f == 4 ? in.T : f == 5 ? in.tke : in.q[f - 6];
+}
+
+// Starts the copies of plane p's raw fields; every thread copies the cells it
+// converts, so its own wait is all the conversion needs.
+template <int ND>
+__device__ __forceinline__ void start_plane(const Grid &G, const In &in, int p, int i0, int j0, double *raw) {
   for (int c = threadIdx.x; c < HP; c += NT) {
-    const int r = c / HX, cc = c % HX;
-    const int gj = j0 - 1 + r, gi = i0 - 1 + cc;
-    const bool inx = gi >= 0 && gi < nx, iny = gj >= 0 && gj < ny;
-    int si = gi, sj = gj;
-    if (!inx && iny) si = G.bc_x == BC_PRECURSOR ? clampi(gi, nx) : wrapi(gi, nx);
-    else if (inx && !iny) sj = G.bc_y == BC_PRECURSOR ? clampi(gj, ny) : wrapi(gj, ny);
-    else if (!inx && !iny) {
-      si = wrapi(gi, nx);
-      sj = wrapi(gj, ny);
-    }
-    int sp = p;
-    bool zhalo = false;
-    if (p < 0 || p >= nz) {
-      if (G.bc_z == BC_WALL) {
-        sp = p < 0 ? 0 : nz - 1;
-        zhalo = true;
-      } else {
-        sp = wrapi(p, nz);
-      }
-    }
-    const size_t q = (size_t(sp) * ny + sj) * nx + si;
-    const double rd = in.rd[q];
-    const double th = pow(rd * G.R_d * in.T[q] / G.C0, G.rgamma) / rd;
-    double val[F];
-    val[iR] = rd;
-    val[iU] = in.u[q];
-    val[iV] = in.v[q];
-    val[iW] = zhalo ? 0.0 : in.w[q];
-    val[iT] = th;
-    val[iK] = fmax(0.0, in.tke[q] / rd);
+    bool zhalo;
+    const size_t q = source_cell(G, c, p, i0, j0, zhalo);
 #pragma unroll
-    for (int t = 0; t < ND; t++) val[6 + t] = in.q[t][q] / rd;
+    for (int f = 0; f < Les<ND>::PRE; f++) copy_async8(raw + f * HP + c, field<ND>(in, f) + q);
+  }
+}
+
+// Primitive fields of the closure (les_closure.h:356-365) of plane p from its
+// copied raw fields; w = 0 and an isentropic density beyond a wall.
+template <int ND>
+__device__ __forceinline__ void finish_plane(const Grid &G, const In &in, int p, int i0, int j0, const double *raw,
+                                             double *ring, uint8_t *flag) {
+  constexpr int F = Les<ND>::F;
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  for (int c = threadIdx.x; c < HP; c += NT) {
+    bool zhalo;
+    const size_t q = source_cell(G, c, p, i0, j0, zhalo);
+    // Flags from the halo array (tile columns past the domain clamp onto its halo).
+    const int hj = min(j0 - 1 + c / HX, G.ny) + 1, hi = min(i0 - 1 + c % HX, G.nx) + 1;
+    flag[c] = __ldg(G.flags + (size_t(p + 1) * (G.ny + 2) + hj) * (G.nx + 2) + hi);
+    double val[F];
+#pragma unroll
+    for (int f = 0; f < F; f++) val[f] = f < Les<ND>::PRE ? raw[f * HP + c] : field<ND>(in, f)[q];
+    const double rd = val[iR], r = 1.0 / rd;
+    const double th = pow(rd * val[iT] * G.Rd_C0, G.rgamma) * r;
+    val[iT] = th;
+    val[iK] = fmax(0.0, val[iK] * r);
+#pragma unroll
+    for (int t = 0; t < ND; t++) val[6 + t] *= r;
     if (zhalo) {
-      const double g = G.gravity ? G.grav : 0.0;
+      val[iW] = 0.0;
       const double rho0_gm1 = pow(rd, G.gamma - 1), theta0_g = pow(th, G.gamma);
-      const double add = g * (G.gamma - 1) * G.dz / (G.gamma * G.C0 * theta0_g);
+      const double add = G.g * (G.gamma - 1) * G.dz / (G.gamma * G.C0 * theta0_g);
       val[iR] = pow(p < 0 ? rho0_gm1 + add : rho0_gm1 - add, G.rgm1);
     }
 #pragma unroll
     for (int f = 0; f < F; f++) ring[f * HP + c] = val[f];
-    // Flags from the halo array (tile columns past the domain clamp onto its halo).
-    const int hj = min(gj, ny) + 1, hi = min(gi, nx) + 1;
-    const double pr = G.prop[(size_t(p + 1) * (ny + 2) + hj) * (nx + 2) + hi];
-    flag[c] = uint8_t((pr == 1 ? F_EQ1 : 0) | (pr > 0 ? F_GT0 : 0) | (pr < 1 ? F_LT1 : 0));
   }
+}
+
+// Mixing length ell = min(0.76 sqrt(K) / N, delta) and sqrt(K), with
+// N = sqrt(g/theta dtheta/dz) where the column is stable, else 0
+// (les_closure.h:96-102).  1/N = theta / sqrt(g theta dtheta/dz) takes one
+// reciprocal square root where the direct form takes two divisions and a
+// square root, the chains this kernel waits on.  (The reference adds 1e-20
+// to N: where N = 0 that is the divisor; beside any other N that leaves
+// 0.76 sqrt(K)/N below delta it is far below N's rounding.)
+__device__ __forceinline__ void mixing(const Grid &G, double K, double t, double dt_dz, double &sK, double &ell) {
+  sK = K > 0 ? K * rsqrt(K) : 0.0;
+  const double b = G.g * t * dt_dz;
+  ell = fmin(0.76 * sK * (b > 0 ? t * rsqrt(b) : 1.e20), G.delta);
 }
 
 // Face quantities (les_closure.h:87-232) for the face between cells A and B
@@ -151,18 +202,21 @@ __device__ __forceinline__ void face_flux(const Grid &G, const double *ring, con
   auto normal = [&](int f) { return (X(f, sB, oB) - X(f, sA, oA)) * rn; };
   // Centred derivative of f along E at A and at B, averaged.
   auto tang = [&](int f, int E) {
-    double a, b;
+    double a, b, r;
     if (E == 0) {
-      a = (X(f, sA, oA + 1) - X(f, sA, oA - 1)) * G.r2dx;
-      b = (X(f, sB, oB + 1) - X(f, sB, oB - 1)) * G.r2dx;
+      a = X(f, sA, oA + 1) - X(f, sA, oA - 1);
+      b = X(f, sB, oB + 1) - X(f, sB, oB - 1);
+      r = G.r2dx;
     } else if (E == 1) {
-      a = (X(f, sA, oA + HX) - X(f, sA, oA - HX)) * G.r2dy;
-      b = (X(f, sB, oB + HX) - X(f, sB, oB - HX)) * G.r2dy;
+      a = X(f, sA, oA + HX) - X(f, sA, oA - HX);
+      b = X(f, sB, oB + HX) - X(f, sB, oB - HX);
+      r = G.r2dy;
     } else {
-      a = (X(f, sp, oA) - X(f, sm, oA)) * G.r2dz;
-      b = (X(f, sp, oB) - X(f, sm, oB)) * G.r2dz;
+      a = X(f, sp, oA) - X(f, sm, oA);
+      b = X(f, sp, oB) - X(f, sm, oB);
+      r = G.r2dz;
     }
-    return 0.5 * (a + b);
+    return (a + b) * (0.5 * r);
   };
   double g[3][3];   // g[c][e]: d(velocity c)/d(direction e)
 #pragma unroll
@@ -176,13 +230,12 @@ __device__ __forceinline__ void face_flux(const Grid &G, const double *ring, con
   const double rho = 0.5 * (X(iR, sA, oA) + X(iR, sB, oB));
   const double K = 0.5 * (X(iK, sA, oA) + X(iK, sB, oB));
   const double t = 0.5 * (X(iT, sA, oA) + X(iT, sB, oB));
-  const double N = dt_dz >= 0 && G.gravity ? sqrt(G.grav / t * dt_dz) : 0.0;
-  const double sK = sqrt(K);
-  const double ell = fmin(0.76 * sK / (N + 1.e-20), G.delta);
+  double sK, ell;
+  mixing(G, K, t, dt_dz, sK, ell);
   const double km = G.total_mult * 0.1 * ell * sK;
-  const double Pr_t = G.delta / (1 + 2 * ell);
+  const double rPr = (1 + 2 * ell) * G.rdelta;
   const double visc = G.dns ? G.nu : fmin(km + G.nu, visc_half);
-  const double visc_th = G.dns ? G.nu : fmin(km / Pr_t + G.nu_Pr, visc_half);
+  const double visc_th = G.dns ? G.nu : fmin(km * rPr + G.nu_Pr, visc_half);
   const double div = g[0][0] + g[1][1] + g[2][2];
   const double mrv = -rho * visc;
 #pragma unroll
@@ -202,14 +255,12 @@ __device__ __forceinline__ double tke_source(const Grid &G, const double *ring, 
   if (!(flag[s * HP + o] & F_LT1)) return 0.0;
   const double rho = X(iR, s, o), K = X(iK, s, o), t = X(iT, s, o);
   const double dt_dz = (X(iT, sp, o) - X(iT, sm, o)) * G.r2dz;
-  const double N = dt_dz >= 0 && G.gravity ? sqrt(G.grav / t * dt_dz) : 0.0;
-  const double sK = sqrt(K);
-  const double ell = fmin(0.76 * sK / (N + 1.e-20), G.delta);
+  double sK, ell;
+  mixing(G, K, t, dt_dz, sK, ell);
   const double km = 0.1 * ell * sK;
-  const double Pr_t = G.delta / (1 + 2 * ell);
   double src = 0.0;
-  if (G.gravity) src += -(G.grav * rho * km) / (t * Pr_t) * dt_dz;
-  src -= G.diss_mult * rho * (0.19 + 0.51 * ell / G.delta) / G.delta * (K * sK);
+  if (G.gravity) src += -(G.grav * rho * km) * ((1 + 2 * ell) * G.rdelta) * dt_dz / t;
+  src -= G.diss_mult * rho * (0.19 + 0.51 * ell * G.rdelta) * G.rdelta * (K * sK);
   // Neighbours inside immersed material are replaced by the cell itself
   // except along a component's own direction.
   const int oxm = (flag[s * HP + o - 1] & F_GT0) ? o : o - 1, oxp = (flag[s * HP + o + 1] & F_GT0) ? o : o + 1;
@@ -238,74 +289,100 @@ __device__ __forceinline__ double tke_source(const Grid &G, const double *ring, 
 __device__ __forceinline__ int slot_of(int p) { return ((p % 3) + 3) % 3; }
 
 template <int ND>
-__global__ void __launch_bounds__(NT) k_les(const Grid G, const In in, const Out out, double dt, double vhx,
-                                            double vhy, double vhz) {
+__global__ void __launch_bounds__(NT, 2) k_les(const Grid G, const In in, const Out out, double dt, double vhx,
+                                               double vhy, double vhz) {
   constexpr int F = Les<ND>::F, NF = Les<ND>::NF;
   extern __shared__ __align__(16) unsigned char smem[];
   double *ring = reinterpret_cast<double *>(smem);                        // [3][F][HP]
-  double *fx = ring + 3 * F * HP;                                          // [NF][TY][TX+1]
-  double *fy = fx + NF * TY * (TX + 1);                                    // [NF][TY+1][TX]
-  uint8_t *flag = reinterpret_cast<uint8_t *>(fy + NF * (TY + 1) * TX);   // [3][HP]
+  double *fy = ring + 3 * F * HP;                                          // [NF][TY+1][TX]
+  double *fxe = fy + NF * (TY + 1) * TX;                                   // [NF][TY]: the tile's last x face
+  double *raw = fxe + NF * TY;                                             // [PRE][HP]
+  uint8_t *flag = reinterpret_cast<uint8_t *>(raw + Les<ND>::PRE * HP);   // [3][HP]
   const int tid = threadIdx.x, tj = tid / TX, ti = tid % TX;
   const int i0 = blockIdx.x * TX, j0 = blockIdx.y * TY;
   const int k0 = blockIdx.z * KC, k1 = min(G.nz, k0 + KC);
   const int i = i0 + ti, j = j0 + tj;
   const bool live = i < G.nx && j < G.ny;
   const int oc = (tj + 1) * HX + (ti + 1);   // this column's offset in the halo tile
-  for (int p = k0 - 1; p <= k0 + 1; p++)
-    load_plane<ND>(G, in, p, i0, j0, ring + slot_of(p) * F * HP, flag + slot_of(p) * HP);
+  for (int p = k0 - 1; p <= k0 + 1; p++) {
+    start_plane<ND>(G, in, p, i0, j0, raw);
+    finish_plane<ND>(G, in, p, i0, j0, raw, ring + slot_of(p) * F * HP, flag + slot_of(p) * HP);
+  }
   __syncthreads();
   double Fb[NF];   // flux through the bottom face of the current cell
   face_flux<ND, 2>(G, ring, flag, slot_of(k0 - 1), tj + 1, ti + 1, slot_of(k0), tj + 1, ti + 1, 0, 0, vhz, Fb);
   for (int k = k0; k < k1; k++) {
     const int sm = slot_of(k - 1), s = slot_of(k), sp = slot_of(k + 1);
-    // x faces (i-1/2 for i = 0..TX) and y faces of this level into shared memory.
-    for (int e = tid; e < TY * (TX + 1) + (TY + 1) * TX; e += NT) {
-      double fl[NF];
-      if (e < TY * (TX + 1)) {
-        const int r = e / (TX + 1), fi = e % (TX + 1);
-        face_flux<ND, 0>(G, ring, flag, s, r + 1, fi, s, r + 1, fi + 1, sm, sp, vhx, fl);
+    const bool more = k + 1 < k1;
+    // The next level's upper plane (k+2 <= k1 <= nz) starts crossing.
+    if (more) start_plane<ND>(G, in, k + 2, i0, j0, raw);
+    const size_t q = (size_t(k) * G.ny + j) * G.nx + i;
+    const double T_old = live ? __ldg(in.T + q) : 0.0;
+    double part[NF], fl[NF];   // part: minus the divergence but for the y faces (and lane 31's high x face)
+    face_flux<ND, 0>(G, ring, flag, s, tj + 1, ti, s, tj + 1, ti + 1, sm, sp, vhx, fl);
 #pragma unroll
-        for (int v = 0; v < NF; v++) fx[v * TY * (TX + 1) + e] = fl[v];
-      } else {
-        const int e2 = e - TY * (TX + 1), fj = e2 / TX, c = e2 % TX;
-        face_flux<ND, 1>(G, ring, flag, s, fj, c + 1, s, fj + 1, c + 1, sm, sp, vhy, fl);
-#pragma unroll
-        for (int v = 0; v < NF; v++) fy[v * (TY + 1) * TX + e2] = fl[v];
-      }
+    for (int v = 0; v < NF; v++) {
+      const double hi = __shfl_down_sync(0xffffffffu, fl[v], 1);
+      part[v] = (fl[v] - (ti < TX - 1 ? hi : 0.0)) * G.rdx;
     }
-    double Ft[NF];
-    face_flux<ND, 2>(G, ring, flag, s, tj + 1, ti + 1, sp, tj + 1, ti + 1, 0, 0, vhz, Ft);
-    const double src = tke_source<ND>(G, ring, flag, s, sm, sp, oc);
+    face_flux<ND, 1>(G, ring, flag, s, tj, ti + 1, s, tj + 1, ti + 1, sm, sp, vhy, fl);
+#pragma unroll
+    for (int v = 0; v < NF; v++) fy[(v * (TY + 1) + tj) * TX + ti] = fl[v];
+    // The faces that close the tile, by two warps that change from level to level.
+    const int wr = (tj + 2 * k) & (TY - 1);
+    if (wr == 0) {
+      face_flux<ND, 1>(G, ring, flag, s, TY, ti + 1, s, TY + 1, ti + 1, sm, sp, vhy, fl);
+#pragma unroll
+      for (int v = 0; v < NF; v++) fy[(v * (TY + 1) + TY) * TX + ti] = fl[v];
+    } else if (wr == 1 && ti < TY) {
+      face_flux<ND, 0>(G, ring, flag, s, ti + 1, TX, s, ti + 1, TX + 1, sm, sp, vhx, fl);
+#pragma unroll
+      for (int v = 0; v < NF; v++) fxe[v * TY + ti] = fl[v];
+    }
+    face_flux<ND, 2>(G, ring, flag, s, tj + 1, ti + 1, sp, tj + 1, ti + 1, 0, 0, vhz, fl);
+#pragma unroll
+    for (int v = 0; v < NF; v++) {
+      part[v] += (Fb[v] - fl[v]) * G.rdz;
+      Fb[v] = fl[v];
+    }
+    part[4] += tke_source<ND>(G, ring, flag, s, sm, sp, oc);
     double cell[F];
 #pragma unroll
     for (int f = 0; f < F; f++) cell[f] = ring[(s * F + f) * HP + oc];
     __syncthreads();   // face fluxes visible; plane k-1 no longer read
-    // The next level's upper plane (k+2 <= k1 <= nz) into the slot of level k-1.
-    if (k + 1 < k1) load_plane<ND>(G, in, k + 2, i0, j0, ring + slot_of(k + 2) * F * HP, flag + slot_of(k + 2) * HP);
+    if (more) finish_plane<ND>(G, in, k + 2, i0, j0, raw, ring + slot_of(k + 2) * F * HP, flag + slot_of(k + 2) * HP);
     if (live) {
-      double tend[NF];
 #pragma unroll
       for (int v = 0; v < NF; v++) {
-        const double ax = fx[v * TY * (TX + 1) + tj * (TX + 1) + ti + 1] - fx[v * TY * (TX + 1) + tj * (TX + 1) + ti];
-        const double ay = fy[v * (TY + 1) * TX + (tj + 1) * TX + ti] - fy[v * (TY + 1) * TX + tj * TX + ti];
-        tend[v] = -ax * G.rdx - ay * G.rdy - (Ft[v] - Fb[v]) * G.rdz;
+        if (ti == TX - 1) part[v] -= fxe[v * TY + tj] * G.rdx;
+        part[v] -= (fy[(v * (TY + 1) + tj + 1) * TX + ti] - fy[(v * (TY + 1) + tj) * TX + ti]) * G.rdy;
       }
-      tend[4] += src;
-      const double rho = cell[iR];
-      const size_t q = (size_t(k) * G.ny + j) * G.nx + i;
-      out.u[q] = (cell[iU] * rho + dt * tend[0]) / rho;
-      out.v[q] = (cell[iV] * rho + dt * tend[1]) / rho;
-      out.w[q] = (cell[iW] * rho + dt * tend[2]) / rho;
-      out.T[q] = G.C0 * pow(cell[iT] * rho + dt * tend[3], G.gamma) / (rho * G.R_d);
-      out.tke[q] = fmax(0.0, cell[iK] * rho + dt * tend[4]);
+      const double rho = cell[iR], rrt = 1.0 / (rho * cell[iT]), dr = dt * (rrt * cell[iT]);
+      out.u[q] = cell[iU] + dr * part[0];
+      out.v[q] = cell[iV] + dr * part[1];
+      out.w[q] = cell[iW] + dr * part[2];
+      // T = C0 (rho theta)^gamma / (rho R_d): the old T times (1 + x)^gamma,
+      // x the relative change of rho theta; the binomial series to x^6 (first
+      // omitted term below 1e-19 for gamma in [1, 2]) unless x is large.
+      const double x = dt * part[3] * rrt;
+      if (G.pser && fabs(x) <= 1. / 256)
+        out.T[q] = T_old + T_old * (x * fma(fma(fma(fma(fma(G.pc[5], x, G.pc[4]), x, G.pc[3]), x, G.pc[2]), x, G.pc[1]),
+                                            x, G.pc[0]));
+      else out.T[q] = G.C0_Rd * pow(cell[iT] * rho + dt * part[3], G.gamma) / rho;
+      out.tke[q] = fmax(0.0, cell[iK] * rho + dt * part[4]);
 #pragma unroll
-      for (int t = 0; t < ND; t++) out.q[t][q] = cell[6 + t] * rho + dt * tend[5 + t];
+      for (int t = 0; t < ND; t++) out.q[t][q] = cell[6 + t] * rho + dt * part[5 + t];
     }
-#pragma unroll
-    for (int v = 0; v < NF; v++) Fb[v] = Ft[v];
-    __syncthreads();   // next plane loaded; face fluxes consumed
+    __syncthreads();   // next plane converted; face fluxes consumed
   }
+}
+
+// The immersed flags of the halo proportion.
+__global__ void k_flags(const double *__restrict__ prop, size_t n, uint8_t *__restrict__ flags) {
+  const size_t e = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (e >= n) return;
+  const double pr = prop[e];
+  flags[e] = uint8_t((pr == 1 ? F_EQ1 : 0) | (pr > 0 ? F_GT0 : 0) | (pr < 1 ? F_LT1 : 0));
 }
 
 // ---------------------------------------------------------------------------
@@ -532,6 +609,7 @@ struct pu_physics {
   cudaStream_t st = nullptr;
   size_t N = 0, NH = 0;
   double *prop = nullptr, *rough = nullptr, *temp = nullptr;   // halo arrays
+  uint8_t *flags = nullptr;      // immersed flags of prop (k_flags)
   double *stage = nullptr;     // (5 + ntr) * N: host views, and the in-place LES output
   double2 *partial = nullptr;  // level-sum partials
   double *mean = nullptr;      // level means [nz][3]
@@ -625,7 +703,14 @@ Grid make_grid(const pu_physics &h) {
   G.diss_mult = c.les_dissipation_mult;
   G.shear_mult = c.les_shear_prod_mult;
   G.delta = std::pow(c.dx * c.dy * c.dz, 1.0 / 3.0);
-  G.prop = h.prop;
+  G.g = G.gravity ? c.grav : 0.0;
+  G.rdelta = 1.0 / G.delta;
+  G.Rd_C0 = c.R_d / c.C0;
+  G.C0_Rd = c.C0 / c.R_d;
+  double b = 1;
+  for (int n = 1; n <= 6; n++) G.pc[n - 1] = b *= (c.gamma_d - (n - 1)) / n;
+  G.pser = c.gamma_d >= 1 && c.gamma_d <= 2;
+  G.flags = h.flags;
   return G;
 }
 
@@ -767,6 +852,8 @@ int pu_physics_create(const pu_physics_config *cfg, const double *imm_prop_h, co
     if (cudaMalloc(&p, h->NH * sizeof(double)) != cudaSuccess) return cleanup(fail(PU_ERR_NOMEM, "cudaMalloc failed"));
     *dst = static_cast<double *>(p);
   }
+  if (cudaMalloc(&p, h->NH) != cudaSuccess) return cleanup(fail(PU_ERR_NOMEM, "cudaMalloc failed"));
+  h->flags = static_cast<uint8_t *>(p);
   if (cudaMalloc(&p, S * h->N * sizeof(double)) != cudaSuccess) return cleanup(fail(PU_ERR_NOMEM, "cudaMalloc failed"));
   h->stage = static_cast<double *>(p);
   if (cudaMalloc(&p, size_t(cfg->nz) * PARTS * 3 * sizeof(double2)) != cudaSuccess)
@@ -784,6 +871,8 @@ int pu_physics_create(const pu_physics_config *cfg, const double *imm_prop_h, co
     if (cudaMemcpyAsync(dst[a], src[a], h->NH * sizeof(double), dev ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice,
                         h->st) != cudaSuccess)
       return cleanup(fail(PU_ERR_CUDA, "copying the immersed halo arrays failed"));
+  k_flags<<<unsigned((h->NH + 255) / 256), 256, 0, h->st>>>(h->prop, h->NH, h->flags);
+  if (cudaGetLastError() != cudaSuccess) return cleanup(fail(PU_ERR_CUDA, "kernel launch failed"));
   if (cudaStreamSynchronize(h->st) != cudaSuccess) return cleanup(fail(PU_ERR_CUDA, "stream synchronize failed"));
   *out = h;
   return PU_OK;
@@ -794,7 +883,7 @@ int pu_physics_destroy(pu_physics *h) {
   {
     Dev g(h->cfg.device);
     cudaStreamSynchronize(h->st);
-    for (void *p : {(void *)h->prop, (void *)h->rough, (void *)h->temp, (void *)h->stage, (void *)h->partial,
+    for (void *p : {(void *)h->prop, (void *)h->rough, (void *)h->temp, (void *)h->flags, (void *)h->stage, (void *)h->partial,
                     (void *)h->mean, (void *)h->tavg_stage, (void *)h->column})
       if (p) cudaFree(p);
     if (h->e0) cudaEventDestroy(h->e0);

@@ -93,6 +93,38 @@ def test_physics_modules_match_oracle(oracle_lib, gpu_lib, kind, device):
     ph.close()
 
 
+@pytest.mark.parametrize("diffused", [0, 1, 2, 3])
+@pytest.mark.parametrize("steep", [False, True])
+def test_les_tracer_counts_and_large_changes(oracle_lib, gpu_lib, diffused, steep):
+    """The closure with 0 to 3 diffused tracers beside TKE on a grid of partial
+    tiles and chunks; steep: temperatures 20 K apart, so that part of the cells
+    change theta by more than the 1/256 up to which T's update is a series."""
+    case, halos, _ = _case("immersed", nx=37, ny=19, nz=21)
+    base = list(case.tracers)
+    wv, tke = base[0], base[1]
+    wv.diffuse = diffused > 0
+    extra = [cases.Tracer("t%d" % q, "", False, False, True) for q in range(max(0, diffused - 1))]
+    case.tracers = [wv, tke] + extra
+    case.tracer_data = np.concatenate([case.tracer_data[:2]] +
+                                      [np.full((1,) + case.rho_d.shape, 0.3 + q) for q in range(len(extra))])
+    st = pyphysics.state_of(case, seed=diffused)
+    rng = np.random.default_rng(diffused)
+    for q in range(len(extra)):
+        st["tracers"][2 + q] += 0.1 * rng.standard_normal(case.rho_d.shape)
+    dt = 0.1
+    if steep:
+        dt = 10.0     # the viscosity at its cap: an eighth of a difference per face
+        st["temp"] = st["temp"] + 20 * rng.uniform(-1, 1, case.rho_d.shape)
+        st["tracers"][1] = 5 + st["tracers"][1]
+    want = pyphysics.Physics(case, "orc", halos).les(st, dt)
+    ph = Physics.from_case(case, halos=halos)
+    got = _run_gpu(ph, "les", st, (dt,), True)
+    ph.close()
+    x = np.abs(want["temp"] / st["temp"] - 1).max()
+    assert (x > 1.4 / 256) if steep else (x < 1 / 256)
+    _check("les/%d/%s" % (diffused, steep), got, want, st)
+
+
 def test_les_out_of_place_equals_in_place(gpu_lib):
     import torch
     case, halos, _ = _case("immersed")
