@@ -53,7 +53,9 @@ __device__ __forceinline__ unsigned long long splitmix64(unsigned long long z) {
 
 // (s - min) / (max - min); all zeros when the range is <= 1e-20 (the
 // reference's normalize keeps scale = 1 there, WenoLimiter.h:85-96).
-// Returns the largest normalised jump between neighbouring entries.
+// Returns the largest normalised jump between neighbouring entries (every
+// operation rounded by itself: the jump decides between the network and the
+// limiter, and all callers must decide alike).
 __device__ __forceinline__ float normalize9(const float (&s)[9], float (&x)[9]) {
   float mn = s[0], mx = s[0];
 #pragma unroll
@@ -64,10 +66,10 @@ __device__ __forceinline__ float normalize9(const float (&s)[9], float (&x)[9]) 
   const float rng = mx - mn;
   const float r = rng > 1e-20f ? 1.f / rng : 0.f;
 #pragma unroll
-  for (int m = 0; m < 9; m++) x[m] = (s[m] - mn) * r;
+  for (int m = 0; m < 9; m++) x[m] = __fmul_rn(s[m] - mn, r);
   float jmp = 0.f;
 #pragma unroll
-  for (int m = 0; m < 8; m++) jmp = fmaxf(jmp, fabsf(x[m + 1] - x[m]));
+  for (int m = 0; m < 8; m++) jmp = fmaxf(jmp, fabsf(__fsub_rn(x[m + 1], x[m])));
   return jmp;
 }
 

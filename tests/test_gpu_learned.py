@@ -184,6 +184,54 @@ def test_learned_fallback_near_immersed(gpu_lib):
     gp.close()
 
 
+@pytest.mark.parametrize("shape", [(32, 16, 20), (40, 24, 12), (64, 4, 24), (33, 17, 16)])
+def test_sorted_queues(gpu_lib, shape):
+    """The kernels sort a tile's (a warp's) stencils into a learned and a
+    fallback queue.  With a network whose output is the ideal weights for any
+    input, the learned edges are the nine-cell linear ones: on a flow that
+    does not vary in z, without gravity, a step with the checks off equals the
+    weno_all = False step (whose z edges are the cell values too) to the
+    rounding of the softmax (1e-6 of each field's range).  With mixed queues
+    every stencil is counted once, and the bits do not depend on the order in
+    which the queues fill."""
+    nx, ny, nz = shape
+    case = cases.small_mixed(nx=nx, ny=ny, nz=nz, immersed=False, ntr=1)
+    case.options["enable_gravity"] = False
+    rd, u, v, w, T, trc = [np.array(a, copy=True) for a in case.coupler_arrays(perturbed=True)]
+    for a in (rd, u, v, T, trc[0]):
+        a[...] = a[nz // 2]
+    w[...] = 0.0
+    theta = np.zeros(mo.N_PARAMS, np.float32)
+    theta[-5:] = np.log(np.array([5, 40, 60, 20, 1]) / 126)
+
+    def step(threshold, weno_all=True):
+        o = dict(case.options, weno_all=weno_all)
+        g = Dycore(nx, ny, nz, 100.0, 100.0, 100.0, case.tracers, o)
+        g.init(rd, u, v, w, T, [trc[0]], None)
+        if threshold is not None:
+            g.learned_set_weights(theta)
+            g.set_weno_mode("learned")
+            g.learned_set_threshold(threshold)
+        g.learned_counts()
+        g.advance(g.compute_time_step(), 1)
+        st, _ = g.get_conserved()
+        counts = g.learned_counts()
+        g.close()
+        return st, counts
+
+    lin, _ = step(None, weno_all=False)
+    st, (nl, _) = step(2.0)
+    assert nl > 0
+    inner = slice(6, nz - 6) if nz > 12 else slice(0, 0)
+    for a, b in zip(st, lin):
+        assert np.abs((a - b)[inner]).max(initial=0) <= 1e-6 * max(np.abs(b).max(), 1e-30)
+    a, ca = step(0.4)
+    b, cb = step(0.4)
+    assert ca == cb and ca[0] > 0 and ca[1] > 0
+    assert sum(ca) == sum(step(0.0)[1]) == sum(step(2.0)[1])
+    assert np.array_equal(a, b)
+
+
 def test_learned_modes_rejected_where_unsupported(gpu_lib):
     case = cases.small_mixed(immersed=False)
     g64 = Dycore.from_case(case, precision="f64")
