@@ -1867,6 +1867,21 @@ __global__ void k_imm_finish(const double *__restrict__ prop, const uint8_t *__r
   mult[idx] = R(pow(pr, power) / tau);
 }
 
+// any[0] = 1 if a cell of the proportion is immersed.
+static __global__ void k_imm_any(const double *__restrict__ prop, size_t N, int *__restrict__ any) {
+  const size_t idx = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  const int hit = __syncthreads_or(idx < N && prop[idx] > 0);
+  if (hit && threadIdx.x == 0) *any = 1;
+}
+
+// top = 1 + the highest level that holds a flag (0: none); top is 0 on entry.
+static __global__ void k_flag_top(const uint8_t *__restrict__ flags, size_t N, size_t NP, int *top) {
+  const size_t idx = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  const int mine = idx < N && flags[idx] ? int(idx / NP) + 1 : 0;
+  const int most = __reduce_max_sync(0xffffffffu, mine);
+  if ((threadIdx.x & 31) == 0 && most > *static_cast<volatile int *>(top)) atomicMax(top, most);
+}
+
 // ---------------------------------------------------------------------------
 // FP64 compensated global integrals.
 // ---------------------------------------------------------------------------

@@ -939,7 +939,7 @@ struct Impl : ImplBase {
       if (rc == PU_OK) rc = dalloc(d1, N);
       if (rc == PU_OK) rc = dalloc(dz, N);
       int *anyp = nullptr;
-      if (rc == PU_OK) rc = dalloc(anyp, 1);
+      if (rc == PU_OK) rc = dalloc(anyp, 2);
       if (rc == PU_OK) rc = imm_prepare(dprop, d0, d1, dz, anyp);
       cudaStreamSynchronize(st);
       for (void *p : {(void *)dprop, (void *)dproj, (void *)d0, (void *)d1, (void *)dz, (void *)anyp})
@@ -953,8 +953,18 @@ struct Impl : ImplBase {
   }
 
   int imm_prepare(const double *dprop, uint8_t *a, uint8_t *b, uint8_t *dzero, int *anyp) {
-    // Any immersed cell at all?
-    PU_CK(cudaMemsetAsync(anyp, 0, sizeof(int), st));
+    // Any immersed cell at all?  Without one there are no flags to build.
+    // (This and the highest flagged level come from the device: scanning a
+    // copy of the flags on the host took about 1 ms per 2.5 M cells.)
+    int h[2] = {0, 0};
+    has_imm = false;
+    imm_kc = 0;
+    PU_CK(cudaMemsetAsync(anyp, 0, sizeof(h), st));
+    k_imm_any<<<blocks(N, 256), 256, 0, st>>>(dprop, N, anyp);
+    PU_LAUNCHED();
+    PU_CK(cudaMemcpyAsync(h, anyp, sizeof(int), cudaMemcpyDeviceToHost, st));
+    PU_CK(cudaStreamSynchronize(st));
+    if (!h[0]) return PU_OK;
     k_dist_init<<<blocks(N, 256), 256, 0, st>>>(dprop, 0, N, a, 10);
     PU_LAUNCHED();
     // a: distance to immersed (cap 10) -> any_immersed10
@@ -980,19 +990,12 @@ struct Impl : ImplBase {
     k_imm_finish<R><<<blocks(N, 256), 256, 0, st>>>(dprop, a, dzero, cfg.immersed_power, N, flags,
                                                     static_cast<R *>(imm_mult));
     PU_LAUNCHED();
-    // has_imm: any flag set (a cell with prop > 0 has distance 0 in `a`).
-    std::vector<uint8_t> hf(N);
-    PU_CK(cudaMemcpyAsync(hf.data(), flags, N, cudaMemcpyDeviceToHost, st));
+    k_flag_top<<<blocks(N, 256), 256, 0, st>>>(flags, N, NP, anyp + 1);
+    PU_LAUNCHED();
+    PU_CK(cudaMemcpyAsync(h, anyp, sizeof(h), cudaMemcpyDeviceToHost, st));
     PU_CK(cudaStreamSynchronize(st));
-    has_imm = false;
-    for (size_t q = 0; q < N && !has_imm; q++) has_imm = (hf[q] & FLAG_IMM) != 0;
-    imm_kc = 0;
-    for (int k = cfg.nz - 1; k >= 0 && !imm_kc; k--)
-      for (size_t q = size_t(k) * NP; q < size_t(k + 1) * NP; q++)
-        if (hf[q]) {
-          imm_kc = k + 1;
-          break;
-        }
+    has_imm = true;
+    imm_kc = h[1];
     return PU_OK;
   }
 
