@@ -16,16 +16,17 @@
 // weighted sum instead of to each weight.
 //
 // The stencil kernels are bound by the FP32 multiply-add pipe, so the count
-// of these operations is what the limiter costs: ~256 per stencil (both
+// of these operations is what the limiter costs: ~240 per stencil (both
 // edges) against ~280 for the earlier form (an LDL^T factorisation of each
 // window's TV and separate edge formulas, 118 operations up to the TVs and
-// edge values where this one takes 94), and ~25 distinct constants instead
+// edge values where this one takes 94; MAP_RATIOS below takes 18 more off), and ~25 distinct constants instead
 // of ~100: the 256x256x128 boundary layer 6.53 -> 6.14 ms per step, the
 // 512x512x128 urban canopy 24.2 -> 22.6 ms, the FP64 build 9 % faster.
 // In FP32 the reciprocals use rcp.approx.ftz; every operand is a normal
-// number there: TV_k^2+1e-20 >= 1e-20, the normalisation sums exceed 1e-20
-// on the branch that divides (the weight sums always), and the map_rs
-// denominator is at least ideal_k^6 > 2e-13.
+// number there (or t^2 = 0, see MAP_RATIOS): TV_k^2+1e-20 >= 1e-20, the
+// normalisation sums exceed 1e-20 on the branch that divides (the weight sums
+// always), and the map_rs denominators, divided by 2000, are at least
+// ideal_k^6/2000 > 1e-16 or 1/2000.
 #pragma once
 
 #include "weno9_tables.cuh"
@@ -172,10 +173,19 @@ __device__ __forceinline__ void weno9_rk(V (&tv)[5], typename Arith<V>::B imm_L,
 // Per-lane constants of one edge: SIDE 0 the left edge, 1 the right edge, 2
 // (float2) the right edge in lane x and the left edge in lane y.
 template <class V, int SIDE>
-__device__ __forceinline__ V ideal_of(int k) {
+__device__ __forceinline__ V ideal_of(int k, double scale = 1.) {
   using namespace pu_weno9;
-  return Arith<V>::c2(SIDE == 0 ? IDEAL_L[k] : IDEAL_R[k], SIDE == 1 ? IDEAL_R[k] : IDEAL_L[k]);
+  return Arith<V>::c2(scale * (SIDE == 0 ? IDEAL_L[k] : IDEAL_R[k]), scale * (SIDE == 1 ? IDEAL_R[k] : IDEAL_L[k]));
 }
+// How many of an edge's five weights are mapped by way of the ratio z = u/t^2,
+//   d + t t^6/(t^6 + 2000 u^3) = d + t/(1 + 2000 z^3),
+// which takes seven multiply-adds and two reciprocals against ten and one.
+// The multiply-add pipe bounds the stencil kernels (79 % busy) and the
+// reciprocals' pipe has room (48 %): on the 256x256x128 boundary layer 0, 2, 3,
+// 4 of five take 24.58, 24.02, 23.94, 24.01 ms for four steps (all five, in a
+// first form of this, were slower than three by 1.5 %).  z is infinite where
+// t = 0, and the weight then the ideal one.
+constexpr int MAP_RATIOS = 3;
 template <class V, int SIDE>
 __device__ __forceinline__ V odd_of() {
   using namespace pu_weno9;
@@ -183,9 +193,10 @@ __device__ __forceinline__ V odd_of() {
 }
 
 // The weights of one edge, negated: -w_k of the ideal-weighted normalised
-// reciprocals, or after map_rs the unnormalised -m_k, whose sum the caller
-// divides by (r: 1/sum(-m_k), or -1).  The signs spare every negated operand
-// in between: with n = -w,  n + d = -(w - d)  and  n n + n = -w (1 - w).
+// reciprocals, or after map_rs the unnormalised -2000 m_k, whose sum the
+// caller divides by (r: 1/sum(-2000 m_k), or -1).  The signs spare every
+// negated operand in between: with n = -w,  n + d = -(w - d)  and
+// n n + n = -w (1 - w) = -u; the factor 2000 spares its multiplication.
 // Both sums always pass the reference's test (> 1e-20): rk_k is at least
 // 1/(1 + 1e-20) when the TVs were normalised (each is then at most 1 up to a
 // rounding) and 1e20 when they were not, so the first is at least the sum of
@@ -204,14 +215,20 @@ __device__ __forceinline__ V weno9_neg_weights(const V (&rk)[5], typename Arith<
     V m[5];
 #pragma unroll
     for (int k = 0; k < 5; k++) {
-      const V dk = ideal_of<V, SIDE>(k);
-      const V t = A::add(n[k], dk);
+      const V t = A::add(n[k], ideal_of<V, SIDE>(k));
       const V t2 = A::mul(t, t);
-      const V t6 = A::mul(A::mul(t2, t2), t2);
       const V u = A::fma(n[k], n[k], n[k]);
-      const V u3 = A::mul(A::mul(u, u), u);
-      const V den = A::fma(A::c(-2000.), u3, t6);
-      m[k] = A::fma(A::mul(t6, t), A::rcp(den), A::neg(dk));
+      const V d2000 = ideal_of<V, SIDE>(k, -2000.);
+      if (k < MAP_RATIOS) {
+        const V z = A::mul(u, A::rcp(A::neg(t2)));
+        const V den = A::fma(A::mul(z, z), z, A::c(1. / 2000.));
+        m[k] = A::fma(t, A::rcp(den), d2000);
+      } else {
+        const V t6 = A::mul(A::mul(t2, t2), t2);
+        const V u3 = A::mul(A::mul(u, u), u);
+        const V den = A::fma(A::c(-1. / 2000.), t6, u3);
+        m[k] = A::fma(A::mul(t6, t), A::rcp(A::neg(den)), d2000);
+      }
     }
     r = A::sel(do_map, A::rcp(sum5(m)), r);
 #pragma unroll
