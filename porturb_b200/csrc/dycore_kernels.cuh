@@ -422,7 +422,7 @@ __device__ __forceinline__ int recon_learned(const Grid<float> &G, uint32_t *sW,
 // (weno_all).  There are F x LINES lines of W+2 cells (positions 0..W+1,
 // cells -1..W); the faces of a line read both edges of the W inner cells, the
 // right edge of position 0 and the left edge of position W+1.  Inner cells go
-// two per thread and iteration (weno9_edges, recon_packed_inner); the two
+// two fields per thread and iteration (recon_packed_inner); the two
 // halo cells of a line go together through the one-edge form
 // (weno9_outer_edges2, recon_outer_pair), which skips the two edges nobody
 // reads.  Per stencil and edge the bits are those of weno9_edges.
@@ -433,74 +433,41 @@ __device__ __forceinline__ int recon_learned(const Grid<float> &G, uint32_t *sW,
 // modification applied; load(f, line, pos, s, imm, any10) is the two
 // together; store(f, line, pos, qL, qR), store_outer(f, line, qR of position
 // 0, qL of position W+1).
-template <int NT, int F, int LINES, int W, bool POS_MAJOR, class Mask, class Vals, class Store>
-__device__ __forceinline__ void recon_packed_inner(Mask mask, Vals vals, Store store) {
-  constexpr int N_IN = F * LINES * W;
-  auto coords = [](int it, int &f, int &line, int &pos) {
-    f = it / (LINES * W);
-    const int q = it % (LINES * W);
-    line = POS_MAJOR ? q % LINES : q / W;
-    pos = (POS_MAJOR ? q / LINES : q % W) + 1;
-  };
-  if constexpr (NT == LINES * W) {
-    // One position per thread: walk its fields in pairs (the same pairs as
-    // below, where stencil it+NT is the next field of stencil it).
-    int f0, line, pos;
-    coords(threadIdx.x, f0, line, pos);
-    unsigned im;
-    bool ax;
-    mask(line, pos, im, ax);
-    const bool il = ((im >> 3) & 1u) != 0, ir = ((im >> 5) & 1u) != 0;
+// need(line, pos): whether a face of the domain reads the position; the warps
+// of a partial tile that have none skip (their edges stay unwritten and are
+// read by faces whose fluxes nobody uses).  In the z kernel this takes the
+// 64x64x48 grid from 31.2 to 27.1 us per launch; in k_xy the test cost more on
+// whole tiles (0.4 %) than it gave on partial ones, so k_xy needs every
+// position.
+template <int NT, int F, int LINES, int W, bool POS_MAJOR, class Need, class Mask, class Vals, class Store>
+__device__ __forceinline__ void recon_packed_inner(Need need, Mask mask, Vals vals, Store store) {
+  static_assert(NT == LINES * W, "one position per thread");
+  const int line = POS_MAJOR ? threadIdx.x % LINES : threadIdx.x / W;
+  const int pos = (POS_MAJOR ? threadIdx.x / LINES : threadIdx.x % W) + 1;
+  if (!need(line, pos)) return;
+  unsigned im;
+  bool ax;
+  mask(line, pos, im, ax);
+  const bool il = ((im >> 3) & 1u) != 0, ir = ((im >> 5) & 1u) != 0;
 #pragma unroll 1
-    for (int f = 0; f + 1 < F; f += 2) {
-      float a[9], b[9];
-      vals(f, line, pos, a, im);
-      vals(f + 1, line, pos, b, im);
-      float2 s2[9], qL, qR;
+  for (int f = 0; f + 1 < F; f += 2) {
+    float a[9], b[9];
+    vals(f, line, pos, a, im);
+    vals(f + 1, line, pos, b, im);
+    float2 s2[9], qL, qR;
 #pragma unroll
-      for (int m = 0; m < 9; m++) s2[m] = make_float2(a[m], b[m]);
-      weno9_edges(s2, qL, qR, bool2{!ax, !ax}, bool2{il, il}, bool2{ir, ir});
-      store(f, line, pos, qL.x, qR.x);
-      store(f + 1, line, pos, qL.y, qR.y);
-    }
-    if constexpr (F % 2 == 1) {
-      // The odd field alone through the scalar limiter (the same bits): a
-      // packed pair with an idle lane would cost the FMA pipe as much as two.
-      float a[9], qL, qR;
-      vals(F - 1, line, pos, a, im);
-      weno9_edges(a, qL, qR, !ax, il, ir);
-      store(F - 1, line, pos, qL, qR);
-    }
-  } else {
-    for (int it = threadIdx.x; it < N_IN; it += 2 * NT) {
-      const int it2 = it + NT;
-      const bool two = it2 < N_IN;
-      int fa, la, pa, fb, lb, pb;
-      coords(it, fa, la, pa);
-      float a[9], b[9];
-      unsigned ia, ib;
-      bool xa, xb;
-      mask(la, pa, ia, xa);
-      vals(fa, la, pa, a, ia);
-      if (two) {
-        coords(it2, fb, lb, pb);
-        mask(lb, pb, ib, xb);
-        vals(fb, lb, pb, b, ib);
-      } else {
-#pragma unroll
-        for (int m = 0; m < 9; m++) b[m] = a[m];
-        ib = ia;
-        xb = xa;
-        fb = fa, lb = la, pb = pa;
-      }
-      float2 s2[9], qL, qR;
-#pragma unroll
-      for (int m = 0; m < 9; m++) s2[m] = make_float2(a[m], b[m]);
-      weno9_edges(s2, qL, qR, bool2{!xa, !xb}, bool2{((ia >> 3) & 1u) != 0, ((ib >> 3) & 1u) != 0},
-                   bool2{((ia >> 5) & 1u) != 0, ((ib >> 5) & 1u) != 0});
-      store(fa, la, pa, qL.x, qR.x);
-      if (two) store(fb, lb, pb, qL.y, qR.y);
-    }
+    for (int m = 0; m < 9; m++) s2[m] = make_float2(a[m], b[m]);
+    weno9_edges(s2, qL, qR, bool2{!ax, !ax}, bool2{il, il}, bool2{ir, ir});
+    store(f, line, pos, qL.x, qR.x);
+    store(f + 1, line, pos, qL.y, qR.y);
+  }
+  if constexpr (F % 2 == 1) {
+    // The odd field alone through the scalar limiter (the same bits): a
+    // packed pair with an idle lane would cost the FMA pipe as much as two.
+    float a[9], qL, qR;
+    vals(F - 1, line, pos, a, im);
+    weno9_edges(a, qL, qR, !ax, il, ir);
+    store(F - 1, line, pos, qL, qR);
   }
 }
 
@@ -522,21 +489,21 @@ __device__ __forceinline__ void recon_outer_pair(int f, int line, Load load, Sto
 // The same lines in FP64 (weno_all): one stencil at a time, a thread walking
 // the fields of one position where there is a thread per position, and the
 // one edge needed from each of the two halo cells that close a line.
-template <int NT, int F, int LINES, int W, bool POS_MAJOR, class Mask, class Vals, class Store>
-__device__ __forceinline__ void recon_f64_inner(Mask mask, Vals vals, Store store) {
-  constexpr int P = LINES * W;
-  for (int p = threadIdx.x; p < P; p += NT) {
-    const int line = POS_MAJOR ? p % LINES : p / W, pos = (POS_MAJOR ? p / LINES : p % W) + 1;
-    unsigned im;
-    bool ax;
-    mask(line, pos, im, ax);
+template <int NT, int F, int LINES, int W, bool POS_MAJOR, class Need, class Mask, class Vals, class Store>
+__device__ __forceinline__ void recon_f64_inner(Need need, Mask mask, Vals vals, Store store) {
+  static_assert(NT == LINES * W, "one position per thread");
+  const int line = POS_MAJOR ? threadIdx.x % LINES : threadIdx.x / W;
+  const int pos = (POS_MAJOR ? threadIdx.x / LINES : threadIdx.x % W) + 1;
+  if (!need(line, pos)) return;
+  unsigned im;
+  bool ax;
+  mask(line, pos, im, ax);
 #pragma unroll 1
-    for (int f = 0; f < F; f++) {
-      double s[9], qL, qR;
-      vals(f, line, pos, s, im);
-      weno9_edges(s, qL, qR, !ax, ((im >> 3) & 1u) != 0, ((im >> 5) & 1u) != 0);
-      store(f, line, pos, qL, qR);
-    }
+  for (int f = 0; f < F; f++) {
+    double s[9], qL, qR;
+    vals(f, line, pos, s, im);
+    weno9_edges(s, qL, qR, !ax, ((im >> 3) & 1u) != 0, ((im >> 5) & 1u) != 0);
+    store(f, line, pos, qL, qR);
   }
 }
 
@@ -553,10 +520,10 @@ __device__ __forceinline__ void recon_f64_outer_pair(int f, int line, Load load,
 }
 
 // Lines of the stencil type: packed pairs in FP32, one by one in FP64.
-template <class R, int NT, int F, int LINES, int W, bool POS_MAJOR, class Mask, class Vals, class Store>
-__device__ __forceinline__ void recon_inner(Mask mask, Vals vals, Store store) {
-  if constexpr (std::is_same<R, float>::value) recon_packed_inner<NT, F, LINES, W, POS_MAJOR>(mask, vals, store);
-  else recon_f64_inner<NT, F, LINES, W, POS_MAJOR>(mask, vals, store);
+template <class R, int NT, int F, int LINES, int W, bool POS_MAJOR, class Need, class Mask, class Vals, class Store>
+__device__ __forceinline__ void recon_inner(Need need, Mask mask, Vals vals, Store store) {
+  if constexpr (std::is_same<R, float>::value) recon_packed_inner<NT, F, LINES, W, POS_MAJOR>(need, mask, vals, store);
+  else recon_f64_inner<NT, F, LINES, W, POS_MAJOR>(need, mask, vals, store);
 }
 template <class R, int W, class Load, class StoreOuter>
 __device__ __forceinline__ void recon_outer(int f, int line, Load load, StoreOuter store_outer) {
@@ -774,7 +741,7 @@ __global__ void __launch_bounds__(TX *TY, LEARNED ? PU_LEARNED_XY_MIN_BLOCKS : (
   if constexpr ((!std::is_same<R, float>::value || PU_PACKED_LIMITER) && !LEARNED) {
     packed = G.weno_all != 0;
     if (packed) {
-      recon_inner<R, NT, F, TY, TX, false>(mask_xc, vals_xc, store_xc);
+      recon_inner<R, NT, F, TY, TX, false>([](int, int) { return true; }, mask_xc, vals_xc, store_xc);
       // Halo pairs of the x lines, and already those of the y lines (kept in
       // YO until the y phase), so that every thread takes one pair here and
       // the y phase is the inner rounds alone.
@@ -858,7 +825,7 @@ __global__ void __launch_bounds__(TX *TY, LEARNED ? PU_LEARNED_XY_MIN_BLOCKS : (
       __syncthreads();   // step 4 has read the flux buffer that holds the queue
       n_fb += recon_learned<NT>(G, sW, queue, qn + 1, F * Sh::EYN, load_y, store_y);
     } else if (packed) {
-      recon_inner<R, NT, F, TX, TY, true>(mask_yc, vals_yc, [&](int f, int cc, int rr, R qL, R qR) {
+      recon_inner<R, NT, F, TX, TY, true>([](int, int) { return true; }, mask_yc, vals_yc, [&](int f, int cc, int rr, R qL, R qR) {
         EL[f * EN + rr * TX + cc] = qL;
         ER[f * EN + rr * TX + cc] = qR;
       });
@@ -1389,6 +1356,7 @@ __global__ void __launch_bounds__(TX *TZ, sizeof(R) == 4 ? PU_ZT_MIN_BLOCKS : PU
   for (int it = tid; it < HZ * TX; it += NT) {
     const int r = it / TX, c = it % TX;
     const int p = k0 - 5 + r, lv = src_level(p);
+    if (p > nz + 4) break;   // beyond the stencils of cell nz, the last a face reads
     const size_t col = row + min(i0 + c, nx - 1);
     R q[S], w[F];
     const int rr = lv - (k0 - 5);   // the halo box's row of level lv
@@ -1457,7 +1425,9 @@ __global__ void __launch_bounds__(TX *TZ, sizeof(R) == 4 ? PU_ZT_MIN_BLOCKS : PU
     mask(c, q, imm, any10);
     vals(f, c, q, s, imm);
   };
-  recon_inner<R, NT, F, TX, TZ, true>(mask, vals, [&](int f, int c, int q, R qL, R qR) {
+  // Cells up to nz - 1, and cell nz in periodic z (face nz reads it).
+  const int top = wall ? nz - 1 : nz;
+  recon_inner<R, NT, F, TX, TZ, true>([&](int, int q) { return k0 - 1 + q <= top; }, mask, vals, [&](int f, int c, int q, R qL, R qR) {
     EL[(f * (TZ + 2) + q) * TX + c] = qL;
     ER[(f * (TZ + 2) + q) * TX + c] = qR;
   });
