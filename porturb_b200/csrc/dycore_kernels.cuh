@@ -123,6 +123,7 @@ struct Grid {
   // a k_xy launch (blockIdx.x, .y count tiles from them): a decomposed tile
   // can run its interior tiles while its halos cross, its edge tiles after.
   int k_first, c_first, i_first, j_first;
+  int late;   // a k_xy launch independent of the kernel before it (see previous_done)
   // Learned WENO weights (kernels instantiated with LEARNED only).
   const uint32_t *ml_frags;     // per-lane operand fragments of the network
   unsigned long long *ml_counts;  // [0] stencils given learned weights, [1] limiter fallbacks
@@ -154,6 +155,27 @@ __device__ __forceinline__ R pow1pm1(const Grid<R> &G, R x) {
       return fmaf(fmaf(fmaf(fmaf(G.pc[4], x, G.pc[3]), x, G.pc[2]), x, G.pc[1]), x, G.pc[0]) * x;
   }
   return pu_expm1(G.gamma * pu_log1p(x));
+}
+
+// ---------------------------------------------------------------------------
+// Programmatic dependent launch.  The stage kernels are launched so that a
+// kernel may start once every block of the one before it has called
+// next_kernel_may_start (or ended): its blocks then fill the SMs that the
+// last wave leaves idle, and the launch itself is hidden.  previous_done waits
+// until the kernel before has completed and its writes are visible (returns at
+// once in a kernel launched the ordinary way).  Every block calls it before it
+// ends, so a kernel that has completed implies that all before it have.
+//   k_xy  waits first, then lets the z kernel start.  A second k_xy launch of
+//         the same stage (the plain levels after the immersed ones) reads and
+//         writes nothing of the first and waits only at its end (Grid::late):
+//         it cannot start before the first has waited.
+//   k_zt  forms its fields and reconstructs from the stage input, which was
+//         complete when k_xy let it start, and waits before it reads the x/y
+//         tendency and writes.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ void previous_done() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void next_kernel_may_start() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
 template <class R, int NTR>
@@ -566,6 +588,8 @@ __global__ void __launch_bounds__(TX *TY, LEARNED ? PU_LEARNED_XY_MIN_BLOCKS : (
   const size_t plane = size_t(k) * G.NP;
   const bool sim2d = G.sim2d != 0;
   if (LEARNED && tid < 2) qn[tid] = 0;
+  if (!G.late) previous_done();
+  next_kernel_may_start();
 
   // 0. TMA staging of the tile's cross (block-uniform decision).  Box origins:
   // the interior at (i0, j0); the 5 rows above at j0-5 (ny-5 for the first
@@ -597,6 +621,7 @@ __global__ void __launch_bounds__(TX *TY, LEARNED ? PU_LEARNED_XY_MIN_BLOCKS : (
           // wait, and give up the tile.
           if (tid == 0) atomicOr(G.err, ERR_TMA);
           tma::mbar_wait(bar, 0);
+          previous_done();
           return;
         }
       }
@@ -886,6 +911,7 @@ __global__ void __launch_bounds__(TX *TY, LEARNED ? PU_LEARNED_XY_MIN_BLOCKS : (
 #pragma unroll
     for (int s = 0; s < S; s++) txy[s * G.N + idx] = tend[s];
   }
+  if (G.late) previous_done();
 }
 
 // Immersed relaxation toward the hydrostatic state and positivity of
@@ -1327,6 +1353,7 @@ __global__ void __launch_bounds__(TX *TZ, sizeof(R) == 4 ? PU_ZT_MIN_BLOCKS : PU
   // periodic halos wrap; dynamics_rk.h:780-797).
   auto src_level = [&](int p) { return (p >= 0 && p < nz) ? p : (wall ? clampi(p, nz) : wrapi(p, nz)); };
 
+  next_kernel_may_start();
   if constexpr (TMA) {
     if (tid == 0) {
       tma::mbar_init(bar);
@@ -1336,7 +1363,6 @@ __global__ void __launch_bounds__(TX *TZ, sizeof(R) == 4 ? PU_ZT_MIN_BLOCKS : PU
       if (pref) {
         tma::mbar_expect(bar + 1, uint32_t(Sh::cell_bytes) * (sn ? 3u : 2u));
         tma::load_4d(QIN, &maps.qin, i0, j, k0, 0, bar + 1);
-        tma::load_4d(TXY, &maps.txy, i0, j, k0, 0, bar + 1);
         if (sn) tma::load_4d(SN, &maps.sn, i0, j, k0, 0, bar + 1);
       }
     }
@@ -1344,7 +1370,12 @@ __global__ void __launch_bounds__(TX *TZ, sizeof(R) == 4 ? PU_ZT_MIN_BLOCKS : PU
     if (!__syncthreads_and(tma::mbar_wait(bar, 0))) {
       // The copy did not complete: report it, give the copies in flight a
       // last bounded wait, and give up the tile.
-      if (tid == 0) atomicOr(G.err, ERR_TMA);
+      // (The cell inputs lack the tendency, which is not asked for yet.)
+      if (tid == 0) {
+        atomicOr(G.err, ERR_TMA);
+        previous_done();
+        if (pref) tma::load_4d(TXY, &maps.txy, i0, j, k0, 0, bar + 1);
+      }
       tma::mbar_wait(bar, 0);
       if (pref) tma::mbar_wait(bar + 1, 0);
       return;
@@ -1383,6 +1414,12 @@ __global__ void __launch_bounds__(TX *TZ, sizeof(R) == 4 ? PU_ZT_MIN_BLOCKS : PU
     }
   }
   __syncthreads();
+
+  // The x/y tendency is the kernel before's: asked for as soon as that is done.
+  if (pref && tid == 0) {
+    previous_done();
+    tma::load_4d(TXY, &maps.txy, i0, j, k0, 0, bar + 1);
+  }
 
   // 2. z edges of the cells at positions q = 0 .. TZ+1 (level k0-1+q).  The
   // immersed bits of a stencil are the levels around its canonical cell cc
@@ -1438,6 +1475,7 @@ __global__ void __launch_bounds__(TX *TZ, sizeof(R) == 4 ? PU_ZT_MIN_BLOCKS : PU
     });
   __syncthreads();
 
+  previous_done();
   // The cell inputs of the finalisation, copied while the block reconstructed.
   if (pref && !__syncthreads_and(tma::mbar_wait(bar + 1, 0))) {
     if (tid == 0) atomicOr(G.err, ERR_TMA);

@@ -51,6 +51,23 @@ struct NvtxRange {
   NvtxRange &operator=(const NvtxRange &) = delete;
 };
 
+// Launches kernel k so that it may start before the kernel ahead of it in the
+// stream has completed (see previous_done in dycore_kernels.cuh).
+template <class... P, class... A>
+inline void launch_early(void (*k)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t st, A &&...a) {
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c = {};
+  c.gridDim = grid;
+  c.blockDim = dim3(threads);
+  c.dynamicSmemBytes = smem;
+  c.stream = st;
+  c.attrs = &at;
+  c.numAttrs = 1;
+  cudaLaunchKernelEx(&c, k, P(a)...);   // a failure is read by PU_LAUNCHED
+}
+
 #define PU_TRY(x)                 \
   do {                            \
     int rc_ = (x);                \
@@ -851,6 +868,7 @@ struct Impl : ImplBase {
     G.c_first = 0;
     G.i_first = 0;
     G.j_first = 0;
+    G.late = 0;
     G.ml_frags = ml_frags;
     G.ml_counts = ml_counts;
     G.ml_jump = ml_jump;
@@ -1077,27 +1095,37 @@ struct Impl : ImplBase {
     if (kl > k0) {
       Grid<R> Gi = Gt;
       Gi.k_first = k0;
-      k_xy<R, NTR, XTX_BIG, XTY_BIG, IMM, false, DEC><<<dim3(bx, by, kl - k0), Sh::NT, Sh::bytes, st>>>(
-          Gi, sin, t, xy_maps[b]);
+      xy_launch(k_xy<R, NTR, XTX_BIG, XTY_BIG, IMM, false, DEC>, !DEC, dim3(bx, by, kl - k0), Sh::NT, Sh::bytes, Gi, sin,
+                t, xy_maps[b]);
       PU_LAUNCHED();
     }
     if (kl < k1) {
       Grid<R> Gp = Gt;
       Gp.k_first = kl;
+      Gp.late = !DEC && kl > k0;
       const dim3 g(bx, by, k1 - kl);
       bool staged = false;
       if constexpr (!DEC && Sp::TMA_FITS) {
         if (xy_tma && static_cast<const void *>(sin) == s[b]) {
-          k_xy<R, NTR, XTX_BIG, XTY_BIG, false, false, false, true><<<g, Sp::NT, Sp::tma_bytes, st>>>(Gp, sin, t,
-                                                                                                    xy_maps[b]);
+          xy_launch(k_xy<R, NTR, XTX_BIG, XTY_BIG, false, false, false, true>, true, g, Sp::NT, Sp::tma_bytes, Gp, sin, t,
+                    xy_maps[b]);
           staged = true;
         }
       }
       if (!staged)
-        k_xy<R, NTR, XTX_BIG, XTY_BIG, false, false, DEC><<<g, Sp::NT, Sp::bytes, st>>>(Gp, sin, t, xy_maps[b]);
+        xy_launch(k_xy<R, NTR, XTX_BIG, XTY_BIG, false, false, DEC>, !DEC, g, Sp::NT, Sp::bytes, Gp, sin, t, xy_maps[b]);
       PU_LAUNCHED();
     }
     return PU_OK;
+  }
+
+  // Decomposed tiles launch their x/y kernel the ordinary way: copies and
+  // events of the halo exchange stand between the stage kernels there.
+  using XyKernel = void (*)(const Grid<R>, const R *, R *, const XyMaps);
+  void xy_launch(XyKernel k, bool early, dim3 g, unsigned nt, size_t bytes, const Grid<R> &G, const R *sin, R *t,
+                 const XyMaps &m) {
+    if (early) launch_early(k, g, nt, bytes, st, G, sin, t, m);
+    else k<<<g, nt, bytes, st>>>(G, sin, t, m);
   }
 
   // The tiled z kernel on z chunks [c0, c1) of ZT_Z levels; FP32 through TMA
@@ -1115,14 +1143,14 @@ struct Impl : ImplBase {
     bool staged = false;
     if constexpr (std::is_same<R, float>::value) {
       if (zt_tma && static_cast<const void *>(sin) == s[b]) {
-        k_zt<R, NTR, ZT_X, ZT_Z, IMM, true><<<g, ZT_X * ZT_Z, Zs::tma_bytes, st>>>(Gc, sin, sn, sout, t, a_n, a_dt,
-                                                                                 n_enforce, zt_maps[b]);
+        launch_early(k_zt<R, NTR, ZT_X, ZT_Z, IMM, true>, g, ZT_X * ZT_Z, Zs::tma_bytes, st, Gc, sin, sn, sout, t, a_n,
+                     a_dt, n_enforce, zt_maps[b]);
         staged = true;
       }
     }
     if (!staged)
-      k_zt<R, NTR, ZT_X, ZT_Z, IMM><<<g, ZT_X * ZT_Z, Zs::bytes, st>>>(Gc, sin, sn, sout, t, a_n, a_dt, n_enforce,
-                                                                     zt_maps[b]);
+      launch_early(k_zt<R, NTR, ZT_X, ZT_Z, IMM>, g, ZT_X * ZT_Z, Zs::bytes, st, Gc, sin, sn, sout, t, a_n, a_dt,
+                   n_enforce, zt_maps[b]);
     PU_LAUNCHED();
     return PU_OK;
   }
@@ -1153,12 +1181,12 @@ struct Impl : ImplBase {
     if (small_tile) {
       using Sh = XYShape<R, NTR, XTX_SM, XTY_SM, IMM, L>;
       dim3 g(blocks(cfg.nx, XTX_SM), blocks(cfg.ny, XTY_SM), cfg.nz);
-      k_xy<R, NTR, XTX_SM, XTY_SM, IMM, L, DEC><<<g, Sh::NT, Sh::bytes, st>>>(G, sin, t, xy_maps[b]);
+      xy_launch(k_xy<R, NTR, XTX_SM, XTY_SM, IMM, L, DEC>, !DEC, g, Sh::NT, Sh::bytes, G, sin, t, xy_maps[b]);
       PU_LAUNCHED();
     } else if (L) {
       using Sh = XYShape<R, NTR, LTX, LTY, IMM, L>;
       dim3 g(blocks(cfg.nx, LTX), blocks(cfg.ny, LTY), cfg.nz);
-      k_xy<R, NTR, LTX, LTY, IMM, L><<<g, Sh::NT, Sh::bytes, st>>>(G, sin, t, xy_maps[b]);
+      xy_launch(k_xy<R, NTR, LTX, LTY, IMM, L>, true, g, Sh::NT, Sh::bytes, G, sin, t, xy_maps[b]);
       PU_LAUNCHED();
     } else if (DEC && dec_edges_only) {
       // The tiles around the interior ones, which ran while the halos crossed.
