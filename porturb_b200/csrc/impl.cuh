@@ -645,12 +645,15 @@ struct Impl : ImplBase {
   static constexpr int LTX = 16, LTY = 16;           // x/y tile of the learned form (ny >= 16)
   static constexpr int XTX_SM = 32, XTY_SM = 4;      // x/y tile for thin domains
   static constexpr int ZT_X = 8, ZT_Z = 32;          // tiled z kernel: columns x levels per block
+  // Its tiles in the overlapped time_step, whose chunks are a tile high: 8x32,
+  // 16x16 or 32x8 (shape 0, 1, 2), all 256 cells.
+  static constexpr int zt_shape(int Z) { return Z == 32 ? 0 : Z == 16 ? 1 : 2; }
   static constexpr int ZTX = 32, ZTY = 4;            // z-march columns per block
   LevelTables<R> lt{};
   bool small_tile = false;
   // TMA staging of the tiled z kernel: maps per stage-input buffer s[b]
   // (halo and cell boxes of s[b], the cell boxes of s[0] and txy).
-  ZtMaps zt_maps[3];
+  ZtMaps zt_maps[3][3];   // [shape][b]
   bool zt_tma = false;
   // TMA staging of the 16x16 x/y kernel (domains without immersed cells):
   // per stage-input buffer s[b] the interior, halo-row and halo-column boxes.
@@ -667,10 +670,13 @@ struct Impl : ImplBase {
       const int nx = cfg.nx, ny = cfg.ny, nz = cfg.nz;
       bool ok = true;
       for (int b = 0; b < 3 && ok; b++) {
-        ok = tma::encode_state(&zt_maps[b].raw, s[b], nx, ny, nz, S, ZT_X, 1, ZT_Z + 10, S) &&
-             tma::encode_state(&zt_maps[b].qin, s[b], nx, ny, nz, S, ZT_X, 1, ZT_Z, S) &&
-             tma::encode_state(&zt_maps[b].sn, s[0], nx, ny, nz, S, ZT_X, 1, ZT_Z, S) &&
-             tma::encode_state(&zt_maps[b].txy, txy, nx, ny, nz, S, ZT_X, 1, ZT_Z, S);
+        auto zt = [&](ZtMaps &m, uint32_t X, uint32_t Z) {
+          return tma::encode_state(&m.raw, s[b], nx, ny, nz, S, X, 1, Z + 10, S) &&
+                 tma::encode_state(&m.qin, s[b], nx, ny, nz, S, X, 1, Z, S) &&
+                 tma::encode_state(&m.sn, s[0], nx, ny, nz, S, X, 1, Z, S) &&
+                 tma::encode_state(&m.txy, txy, nx, ny, nz, S, X, 1, Z, S);
+        };
+        ok = zt(zt_maps[0][b], 8, 32) && zt(zt_maps[1][b], 16, 16) && zt(zt_maps[2][b], 32, 8);
       }
       zt_tma = ok;
       ok = XTX_BIG == 16 && XTY_BIG == 16;
@@ -742,6 +748,21 @@ struct Impl : ImplBase {
     return configure();
   }
 
+  template <int X, int Z>
+  int zt_configure() {
+    PU_CK(cudaFuncSetAttribute(k_zt<R, NTR, X, Z, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               int(ZTShape<R, NTR, X, Z, false>::bytes)));
+    PU_CK(cudaFuncSetAttribute(k_zt<R, NTR, X, Z, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               int(ZTShape<R, NTR, X, Z, true>::bytes)));
+    if constexpr (std::is_same<R, float>::value) {
+      PU_CK(cudaFuncSetAttribute(k_zt<R, NTR, X, Z, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 int(ZTShape<R, NTR, X, Z, false>::tma_bytes)));
+      PU_CK(cudaFuncSetAttribute(k_zt<R, NTR, X, Z, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 int(ZTShape<R, NTR, X, Z, true>::tma_bytes)));
+    }
+    return PU_OK;
+  }
+
   // Kernel attributes (no allocation).
   int configure() {
     small_tile = cfg.ny < 16;
@@ -769,15 +790,10 @@ struct Impl : ImplBase {
                                int(ZShape<R, NTR, ZTX, ZTY>::bytes)));
     PU_CK(cudaFuncSetAttribute(k_z<R, NTR, ZTX, ZTY, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                int(ZShape<R, NTR, ZTX, ZTY>::bytes)));
-    PU_CK(cudaFuncSetAttribute(k_zt<R, NTR, ZT_X, ZT_Z, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               int(ZTShape<R, NTR, ZT_X, ZT_Z, false>::bytes)));
-    PU_CK(cudaFuncSetAttribute(k_zt<R, NTR, ZT_X, ZT_Z, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               int(ZTShape<R, NTR, ZT_X, ZT_Z, true>::bytes)));
+    PU_TRY((zt_configure<ZT_X, ZT_Z>()));
     if constexpr (std::is_same<R, float>::value) {
-      PU_CK(cudaFuncSetAttribute(k_zt<R, NTR, ZT_X, ZT_Z, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 int(ZTShape<R, NTR, ZT_X, ZT_Z, false>::tma_bytes)));
-      PU_CK(cudaFuncSetAttribute(k_zt<R, NTR, ZT_X, ZT_Z, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 int(ZTShape<R, NTR, ZT_X, ZT_Z, true>::tma_bytes)));
+      PU_TRY((zt_configure<16, 16>()));
+      PU_TRY((zt_configure<32, 8>()));
       if constexpr (XYShape<R, NTR, XTX_BIG, XTY_BIG, false>::TMA_FITS)
         PU_CK(cudaFuncSetAttribute(k_xy<R, NTR, XTX_BIG, XTY_BIG, false, false, false, true>,
                                    cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1128,45 +1144,46 @@ struct Impl : ImplBase {
     else k<<<g, nt, bytes, st>>>(G, sin, t, m);
   }
 
-  // The tiled z kernel on z chunks [c0, c1) of ZT_Z levels; FP32 through TMA
-  // where the stage input is s[b] (the cell maps of sn and txy are the same
-  // for every b).
-  template <bool IMM>
+  // The tiled z kernel with X x Z tiles on z chunks [c0, c1) of Z levels; FP32
+  // through TMA where the stage input is s[b] (the cell maps of sn and txy are
+  // the same for every b).
+  template <bool IMM, int X, int Z>
   int zt_launch(const Grid<R> &G, const R *sin, const R *sn, R *sout, R a_n, R a_dt, int n_enforce, int b, int c0,
                 int c1) {
-    using Zs = ZTShape<R, NTR, ZT_X, ZT_Z, IMM>;
+    using Zs = ZTShape<R, NTR, X, Z, IMM>;
     if (c1 <= c0) return PU_OK;
     const R *t = static_cast<const R *>(txy);
     Grid<R> Gc = G;
     Gc.c_first = c0;
-    const dim3 g(blocks(cfg.nx, ZT_X), unsigned(cfg.ny), unsigned(c1 - c0));
+    const ZtMaps &maps = zt_maps[zt_shape(Z)][b];
+    const dim3 g(blocks(cfg.nx, X), unsigned(cfg.ny), unsigned(c1 - c0));
     bool staged = false;
     if constexpr (std::is_same<R, float>::value) {
       if (zt_tma && static_cast<const void *>(sin) == s[b]) {
-        launch_early(k_zt<R, NTR, ZT_X, ZT_Z, IMM, true>, g, ZT_X * ZT_Z, Zs::tma_bytes, st, Gc, sin, sn, sout, t, a_n,
-                     a_dt, n_enforce, zt_maps[b]);
+        launch_early(k_zt<R, NTR, X, Z, IMM, true>, g, X * Z, Zs::tma_bytes, st, Gc, sin, sn, sout, t, a_n, a_dt,
+                     n_enforce, maps);
         staged = true;
       }
     }
     if (!staged)
-      launch_early(k_zt<R, NTR, ZT_X, ZT_Z, IMM>, g, ZT_X * ZT_Z, Zs::bytes, st, Gc, sin, sn, sout, t, a_n, a_dt,
-                   n_enforce, zt_maps[b]);
+      launch_early(k_zt<R, NTR, X, Z, IMM>, g, X * Z, Zs::bytes, st, Gc, sin, sn, sout, t, a_n, a_dt, n_enforce, maps);
     PU_LAUNCHED();
     return PU_OK;
   }
 
-  // The tiled z kernel (z_tiled) on z chunks [c0, c1): chunks below ci take
-  // the immersed kernel.  Chunk c reads levels 32c-5 .. 32c+36, so it is plain
-  // once 32c-5 reaches the first level no flag holds; a periodic z wraps
-  // flagged levels into the top chunk, so every chunk stays immersed there.
-  template <bool IMM>
+  // The tiled z kernel (z_tiled) on z chunks [c0, c1) of Z levels: chunks
+  // below ci take the immersed kernel.  Chunk c reads levels Zc-5 .. Zc+Z+4,
+  // so it is plain once Zc-5 reaches the first level no flag holds; a periodic
+  // z wraps flagged levels into the top chunk, so every chunk stays immersed
+  // there.
+  template <bool IMM, int X = ZT_X, int Z = ZT_Z>
   int zt_chunks(const Grid<R> &G, const R *sin, const R *sn, R *sout, R a_n, R a_dt, int n_enforce, int b, int c0,
                 int c1) {
-    const int nch = int(blocks(cfg.nz, ZT_Z));
-    const int ci0 = !IMM ? 0 : (cfg.bc_z == PU_BC_WALL ? std::min(nch, (imm_levels() + 5 + ZT_Z - 1) / ZT_Z) : nch);
+    const int nch = int(blocks(cfg.nz, Z));
+    const int ci0 = !IMM ? 0 : (cfg.bc_z == PU_BC_WALL ? std::min(nch, (imm_levels() + 5 + Z - 1) / Z) : nch);
     const int ci = std::min(std::max(ci0, c0), c1);
-    PU_TRY((zt_launch<IMM>(G, sin, sn, sout, a_n, a_dt, n_enforce, b, c0, ci)));
-    return zt_launch<false>(G, sin, sn, sout, a_n, a_dt, n_enforce, b, ci, c1);
+    PU_TRY((zt_launch<IMM, X, Z>(G, sin, sn, sout, a_n, a_dt, n_enforce, b, c0, ci)));
+    return zt_launch<false, X, Z>(G, sin, sn, sout, a_n, a_dt, n_enforce, b, ci, c1);
   }
 
   // One SSPRK3 stage: the x/y kernel (DEC: a decomposed tile reading its
@@ -1272,7 +1289,7 @@ struct Impl : ImplBase {
   // ---- time_step with the host copies overlapped ----
   // On host coupler arrays the copies in and out move 2 x 8 S N bytes over the
   // host link, as long as several steps on large grids.  Here the call runs
-  // as a wavefront over chunks of ZT_Z levels: the input crosses chunk by
+  // as a wavefront over chunks of 8, 16 or 32 levels: the input crosses chunk by
   // chunk on a copy stream, and stage g (1 .. 3 nsteps; 0 = the chunk's
   // conversion and enforcement) runs on chunk c once stage g-1 has run on
   // chunks c-1, c and c+1 (the z stencils reach 5 levels into each
@@ -1288,7 +1305,7 @@ struct Impl : ImplBase {
   // Every cell gets the kernels and inputs of load_state + advance +
   // store_state, so the results are the same bits.  FP32 with the tiled z
   // kernel, walls in z (a periodic z couples the top and bottom chunks), at
-  // least two chunks; the config's serial_io turns it off.
+  // least 64 levels; the config's serial_io turns it off.
   bool io_overlap(const pu_state_view *v) const {
     if constexpr (!std::is_same<R, float>::value) {
       return false;
@@ -1309,13 +1326,14 @@ struct Impl : ImplBase {
         return PU_ERR_INVALID;
       }
     if (!cs) PU_CK(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
-    const int nch = int(blocks(cfg.nz, ZT_Z));
+    const int Z = io_levels(nsteps), nch = int(blocks(cfg.nz, Z));
     while (io_ev.size() < size_t(2 * nch + 1)) {
       cudaEvent_t e;
       PU_CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
       io_ev.push_back(e);
     }
-    const int rc = has_imm ? time_step_io<true>(host, dt, nsteps, nch) : time_step_io<false>(host, dt, nsteps, nch);
+    const int rc = has_imm ? time_step_chunks<true>(host, dt, nsteps, Z, nch)
+                           : time_step_chunks<false>(host, dt, nsteps, Z, nch);
     // No copy into or out of the caller's arrays outlives the call.
     const cudaError_t e = cudaStreamSynchronize(cs);
     if (rc) return rc;
@@ -1326,7 +1344,33 @@ struct Impl : ImplBase {
     return check_err();
   }
 
+  // Levels per chunk.  While the first chunks cross and while the last ones
+  // drain the device idles, the less the thinner the chunks; thin tiles cost
+  // the z kernel more halo (its launch on the 256x256x128 boundary layer takes
+  // ~4 % longer with 16 levels and ~20 % with 8), and a chunk must fill the
+  // device.  Measured, ms per call with 32 / 16 / 8 levels:
+  //   256x256x128   1 step 18.7 / 17.4 / 17.8   4 steps 36.7 / 31.4 / 29.8
+  //                 6 steps 48.5 / 43.7 / 42.7  10 steps 72.4 / 68.1 / 68.6
+  //   192x128x96    2 steps 7.68 / 6.40 / 5.78  4 steps 11.1 / 10.1 / 9.9
+  //                 6 steps 14.6 / 13.8 / 14.0
+  //   128x128x128   4 steps 9.57 / 8.69 / 8.77  10 steps 18.9 / 18.8 / 20.1
+  int io_levels(int nsteps) const {
+    const unsigned tiles = blocks(cfg.nx, XTX_BIG) * blocks(cfg.ny, XTY_BIG);
+    if (tiles < 64) return 32;
+    return nsteps >= 2 && tiles >= 96 && nsteps <= (tiles >= 256 ? 8 : 4) ? 8 : 16;
+  }
+
   template <bool IMM>
+  int time_step_chunks(double *const *host, double dt, int nsteps, int Z, int nch) {
+    if constexpr (std::is_same<R, float>::value) {
+      if (Z == 32) return time_step_io<IMM, 8, 32>(host, dt, nsteps, nch);
+      if (Z == 16) return time_step_io<IMM, 16, 16>(host, dt, nsteps, nch);
+      return time_step_io<IMM, 32, 8>(host, dt, nsteps, nch);
+    }
+    return PU_ERR_UNSUPPORTED;   // io_overlap is FP32
+  }
+
+  template <bool IMM, int X, int Z>
   int time_step_io(double *const *host, double dt, int nsteps, int nch) {
     NvtxRange range("pu:time_step_overlapped");
     const Grid<R> G = grid();
@@ -1340,7 +1384,7 @@ struct Impl : ImplBase {
     cp.T = co.T = staging + 4 * N;
     for (int t = 0; t < 8; t++) cp.tr[t] = co.tr[t] = t < NTR ? staging + size_t(5 + t) * N : nullptr;
     cudaEvent_t *ein = io_ev.data(), *eout = ein + nch, start = ein[2 * nch];
-    auto lev = [&](int c) { return std::min(cfg.nz, c * ZT_Z); };
+    auto lev = [&](int c) { return std::min(cfg.nz, c * Z); };
     const int last = 3 * nsteps;
     // The copy stream starts after the work queued so far (the staging
     // buffer is free then).
@@ -1369,8 +1413,8 @@ struct Impl : ImplBase {
       const R a_dt = m == 0 ? R(dt) : (m == 1 ? R(1. / 4. * dt) : R(2. / 3. * dt));
       const int n_enforce = (m == 2 && g != last) ? 2 : 1;
       PU_TRY((xy_levels<IMM>(G, sb[m], m, lev(c), lev(c + 1))));
-      PU_TRY((zt_chunks<IMM>(G, sb[m], m == 0 ? nullptr : sb[0], sb[(m + 1) % 3], a_n, a_dt, n_enforce, m, c,
-                             c + 1)));
+      PU_TRY((zt_chunks<IMM, X, Z>(G, sb[m], m == 0 ? nullptr : sb[0], sb[(m + 1) % 3], a_n, a_dt, n_enforce, m, c,
+                                   c + 1)));
       if (g == last) {
         k_store_coupler<R, NTR><<<nb, 256, 0, st>>>(co, thermo(), rho_off, rt_off, N, NP, sb[0], e0, e1);
         PU_LAUNCHED();

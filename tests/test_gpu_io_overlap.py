@@ -86,6 +86,25 @@ def test_overlapped_time_step_same_bits_at_config_size(gpu_lib):
     assert np.array_equal(st0, st1) and np.array_equal(tr0, tr1)
 
 
+@pytest.mark.parametrize("name,make,factor", [
+    ("16_levels", lambda: cases.abl_neutral(nx=128, ny=128, nz=66), 1.0),
+    ("16_levels_many_steps", lambda: cases.abl_neutral(nx=144, ny=112, nz=64), 5.0),
+    ("8_levels", lambda: cases.abl_neutral(nx=192, ny=128, nz=70), 2.5),
+    ("8_levels_immersed", lambda: cases.urban_canopy(nx=180, ny=136, nz=73, dx=2.0), 2.5),
+])
+def test_thin_chunks_same_bits(name, make, factor, gpu_lib):
+    """Grids of 63 and more 16x16 tiles run in chunks of 16 or 8 levels (16x16
+    and 32x8 z tiles), with last chunks of 1 to 6 levels: the bits of the
+    serial form."""
+    case = make()
+    n1, l1, out1, st1, tr1 = _call(case, True, factor, False)
+    n0, l0, out0, st0, tr0 = _call(case, False, factor, False)
+    assert n0 == n1 and l0 > l1
+    for q, (a, b) in enumerate(zip(out0, out1)):
+        assert np.array_equal(a, b), (name, q, np.abs(a - b).max())
+    assert np.array_equal(st0, st1) and np.array_equal(tr0, tr1)
+
+
 @pytest.mark.parametrize("name,make", [
     ("periodic_z", lambda: cases.small_mixed(nx=32, ny=32, nz=64, bc_z="periodic")),
     ("nz_48", lambda: cases.abl_neutral(nx=32, ny=32, nz=48)),
