@@ -1569,13 +1569,14 @@ struct Thermo {
 };
 
 // Cells [e0, e1) (whole levels) of the coupler arrays into the state.
-template <class R, int NTR>
-__global__ void k_load_coupler(CouplerPtrs cp, Thermo th, const double *__restrict__ rho_off,
-                               const double *__restrict__ rt_off, size_t N, size_t NP, R *__restrict__ s, size_t e0,
-                               size_t e1) {
-  const size_t idx = e0 + size_t(blockIdx.x) * blockDim.x + threadIdx.x;
+// ENFORCE: followed by the enforcement that opens the first step (k_enforce),
+// as time_step runs the two: one pass over the state and one launch fewer.
+template <class R, int NTR, bool ENFORCE = false, bool IMM = false>
+__global__ void k_load_coupler(const Grid<R> G, CouplerPtrs cp, Thermo th, const double *__restrict__ rho_off,
+                               const double *__restrict__ rt_off, R *__restrict__ s, size_t e0, size_t e1) {
+  const size_t N = G.N, idx = e0 + size_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (idx >= e1) return;
-  const int k = int(idx / NP);
+  const int k = int(idx / G.NP);
   const double rd = cp.rho_d[idx], u = cp.u[idx], v = cp.v[idx], w = cp.w[idx], temp = cp.T[idx];
   const double rho_v = cp.tr[th.idWV][idx];
   const double press = rd * th.R_d * temp + rho_v * th.R_v * temp;
@@ -1584,13 +1585,17 @@ __global__ void k_load_coupler(CouplerPtrs cp, Thermo th, const double *__restri
   for (int t = 0; t < NTR; t++)
     if ((th.adds_mass >> t) & 1u) rho += cp.tr[t][idx];
   const double theta = pow(press / th.C0, 1. / th.gamma) / rho;
-  s[0 * N + idx] = R(rho - rho_off[k]);
-  s[1 * N + idx] = R(rho * u);
-  s[2 * N + idx] = R(rho * v);
-  s[3 * N + idx] = R(rho * w);
-  s[4 * N + idx] = R(rho * theta - rt_off[k]);
+  R q[5 + NTR];
+  q[0] = R(rho - rho_off[k]);
+  q[1] = R(rho * u);
+  q[2] = R(rho * v);
+  q[3] = R(rho * w);
+  q[4] = R(rho * theta - rt_off[k]);
 #pragma unroll
-  for (int t = 0; t < NTR; t++) s[(5 + t) * N + idx] = R(cp.tr[t][idx]);
+  for (int t = 0; t < NTR; t++) q[5 + t] = R(cp.tr[t][idx]);
+  if constexpr (ENFORCE) enforce_cell<R, NTR, IMM>(G, q, idx, k);
+#pragma unroll
+  for (int f = 0; f < 5 + NTR; f++) s[f * N + idx] = q[f];
 }
 
 // Cells [e0, e1) (whole levels) of the state into the coupler arrays.

@@ -1037,8 +1037,19 @@ struct Impl : ImplBase {
     NvtxRange range("pu:load_state");
     CouplerPtrs cp;
     PU_TRY(device_view(v, cp));
-    k_load_coupler<R, NTR><<<blocks(N, 256), 256, 0, st>>>(cp, thermo(), rho_off, rt_off, N, NP,
-                                                           static_cast<R *>(s[0]), 0, N);
+    return load_cells<false>(cp, 0, N);
+  }
+
+  // Cells [e0, e1) of device coupler arrays into the state (ENFORCE: and the
+  // enforcement that opens a step).
+  template <bool ENFORCE>
+  int load_cells(const CouplerPtrs &cp, size_t e0, size_t e1) {
+    R *s0 = static_cast<R *>(s[0]);
+    const unsigned nb = blocks(e1 - e0, 256);
+    if (ENFORCE && has_imm)
+      k_load_coupler<R, NTR, ENFORCE, true><<<nb, 256, 0, st>>>(grid(), cp, thermo(), rho_off, rt_off, s0, e0, e1);
+    else
+      k_load_coupler<R, NTR, ENFORCE><<<nb, 256, 0, st>>>(grid(), cp, thermo(), rho_off, rt_off, s0, e0, e1);
     PU_LAUNCHED();
     return PU_OK;
   }
@@ -1239,14 +1250,16 @@ struct Impl : ImplBase {
   }
 
   template <bool IMM, bool LRN>
-  int advance_t(double dt, int nsteps) {
+  int advance_t(double dt, int nsteps, bool enforced) {
     NvtxRange range("pu:advance");
     const Grid<R> G = grid();
     R *s0 = static_cast<R *>(s[0]), *s1 = static_cast<R *>(s[1]), *s2 = static_cast<R *>(s[2]);
-    cudaEvent_t e0 = prof_begin();
-    k_enforce<R, NTR, IMM><<<blocks(N, 256), 256, 0, st>>>(G, s0, 0, N);
-    PU_LAUNCHED();
-    prof_end(2, e0);
+    if (!enforced) {
+      cudaEvent_t e0 = prof_begin();
+      k_enforce<R, NTR, IMM><<<blocks(N, 256), 256, 0, st>>>(G, s0, 0, N);
+      PU_LAUNCHED();
+      prof_end(2, e0);
+    }
     for (int n = 0; n < nsteps; n++) {
       // Shu-Osher SSPRK(3,3) (dynamics_rk.h:308-360): s1 = s0 + dt L(s0);
       // s2 = 3/4 s0 + 1/4 (s1 + dt L(s1)); s0 <- 1/3 s0 + 2/3 (s2 + dt L(s2)).
@@ -1282,8 +1295,15 @@ struct Impl : ImplBase {
         }
       return PU_OK;
     }
-    if (learned_active()) return has_imm ? advance_t<true, true>(dt, nsteps) : advance_t<false, true>(dt, nsteps);
-    return has_imm ? advance_t<true, false>(dt, nsteps) : advance_t<false, false>(dt, nsteps);
+    return advance_whole(dt, nsteps, false);
+  }
+
+  // The steps of an undecomposed domain; enforced: the state already went
+  // through the enforcement that opens the first one.
+  int advance_whole(double dt, int nsteps, bool enforced) {
+    if (learned_active())
+      return has_imm ? advance_t<true, true>(dt, nsteps, enforced) : advance_t<false, true>(dt, nsteps, enforced);
+    return has_imm ? advance_t<true, false>(dt, nsteps, enforced) : advance_t<false, false>(dt, nsteps, enforced);
   }
 
   // ---- time_step with the host copies overlapped ----
@@ -1317,7 +1337,14 @@ struct Impl : ImplBase {
   }
 
   int time_step(pu_state_view *v, double dt, int nsteps) override {
-    if (nsteps <= 0 || !io_overlap(v)) return ImplBase::time_step(v, dt, nsteps);
+    if (nsteps <= 0 || dc.on) return ImplBase::time_step(v, dt, nsteps);
+    if (!io_overlap(v)) {
+      CouplerPtrs cp;
+      PU_TRY(device_view(v, cp));
+      PU_TRY(load_cells<true>(cp, 0, N));
+      PU_TRY(advance_whole(dt, nsteps, true));
+      return store_state(v);
+    }
     double *host[5 + NTR] = {v->rho_d, v->uvel, v->vvel, v->wvel, v->temp};
     for (int t = 0; t < NTR; t++) host[5 + t] = v->tracers[t];
     for (int a = 0; a < 5 + NTR; a++)
@@ -1402,11 +1429,7 @@ struct Impl : ImplBase {
                                 cudaMemcpyHostToDevice, cs));
         PU_CK(cudaEventRecord(ein[c], cs));
         PU_CK(cudaStreamWaitEvent(st, ein[c], 0));
-        k_load_coupler<R, NTR><<<nb, 256, 0, st>>>(cp, thermo(), rho_off, rt_off, N, NP, sb[0], e0, e1);
-        PU_LAUNCHED();
-        k_enforce<R, NTR, IMM><<<nb, 256, 0, st>>>(G, sb[0], e0, e1);
-        PU_LAUNCHED();
-        return PU_OK;
+        return load_cells<true>(cp, e0, e1);
       }
       const int m = (g - 1) % 3;   // 0: s1 = s0 + dt L(s0); 1: s2 from s1; 2: s0 from s2
       const R a_n = m == 0 ? R(0) : (m == 1 ? R(3. / 4.) : R(1. / 3.));
