@@ -74,6 +74,13 @@ namespace pu {
 #ifndef PU_ZT_MIN_BLOCKS_F64
 #define PU_ZT_MIN_BLOCKS_F64 2
 #endif
+// Threads per cell of the stage kernels where a launch has so few blocks that
+// they are resident at once with that many: the time of such a launch is that
+// of one block, and that mostly the reconstruction of the fields one pair after
+// the other (FP32, plain weights).
+#ifndef PU_SMALL_SPLIT
+#define PU_SMALL_SPLIT 4
+#endif
 #ifndef PU_LEARNED_Z_MIN_BLOCKS
 #define PU_LEARNED_Z_MIN_BLOCKS 3
 #endif
@@ -461,18 +468,22 @@ __device__ __forceinline__ int recon_learned(const Grid<float> &G, uint32_t *sW,
 // 64x64x48 grid from 31.2 to 27.1 us per launch; in k_xy the test cost more on
 // whole tiles (0.4 %) than it gave on partial ones, so k_xy needs every
 // position.
-template <int NT, int F, int LINES, int W, bool POS_MAJOR, class Need, class Mask, class Vals, class Store>
+// SPLIT: that many threads share a position, each taking every SPLIT-th pair of
+// its fields (the blocks of small grids, see PU_SMALL_SPLIT).
+template <int NT, int SPLIT, int F, int LINES, int W, bool POS_MAJOR, class Need, class Mask, class Vals, class Store>
 __device__ __forceinline__ void recon_packed_inner(Need need, Mask mask, Vals vals, Store store) {
-  static_assert(NT == LINES * W, "one position per thread");
-  const int line = POS_MAJOR ? threadIdx.x % LINES : threadIdx.x / W;
-  const int pos = (POS_MAJOR ? threadIdx.x / LINES : threadIdx.x % W) + 1;
+  constexpr int P = LINES * W;
+  static_assert(NT == P * SPLIT, "SPLIT threads per position");
+  const int p = threadIdx.x % P, part = SPLIT == 1 ? 0 : threadIdx.x / P;
+  const int line = POS_MAJOR ? p % LINES : p / W;
+  const int pos = (POS_MAJOR ? p / LINES : p % W) + 1;
   if (!need(line, pos)) return;
   unsigned im;
   bool ax;
   mask(line, pos, im, ax);
   const bool il = ((im >> 3) & 1u) != 0, ir = ((im >> 5) & 1u) != 0;
 #pragma unroll 1
-  for (int f = 0; f + 1 < F; f += 2) {
+  for (int f = 2 * part; f + 1 < F; f += 2 * SPLIT) {
     float a[9], b[9];
     vals(f, line, pos, a, im);
     vals(f + 1, line, pos, b, im);
@@ -486,6 +497,7 @@ __device__ __forceinline__ void recon_packed_inner(Need need, Mask mask, Vals va
   if constexpr (F % 2 == 1) {
     // The odd field alone through the scalar limiter (the same bits): a
     // packed pair with an idle lane would cost the FMA pipe as much as two.
+    if (part != F / 2 % SPLIT) return;
     float a[9], qL, qR;
     vals(F - 1, line, pos, a, im);
     weno9_edges(a, qL, qR, !ax, il, ir);
@@ -542,9 +554,11 @@ __device__ __forceinline__ void recon_f64_outer_pair(int f, int line, Load load,
 }
 
 // Lines of the stencil type: packed pairs in FP32, one by one in FP64.
-template <class R, int NT, int F, int LINES, int W, bool POS_MAJOR, class Need, class Mask, class Vals, class Store>
+template <class R, int NT, int SPLIT, int F, int LINES, int W, bool POS_MAJOR, class Need, class Mask, class Vals,
+          class Store>
 __device__ __forceinline__ void recon_inner(Need need, Mask mask, Vals vals, Store store) {
-  if constexpr (std::is_same<R, float>::value) recon_packed_inner<NT, F, LINES, W, POS_MAJOR>(need, mask, vals, store);
+  if constexpr (std::is_same<R, float>::value)
+    recon_packed_inner<NT, SPLIT, F, LINES, W, POS_MAJOR>(need, mask, vals, store);
   else recon_f64_inner<NT, F, LINES, W, POS_MAJOR>(need, mask, vals, store);
 }
 template <class R, int W, class Load, class StoreOuter>
@@ -561,10 +575,13 @@ __device__ __forceinline__ void recon_outer(int f, int line, Load load, StoreOut
 // sin), the halo rows and columns wrapping periodically box by box; tiles at
 // a precursor edge, partial tiles and halo boxes that would straddle the
 // domain's edge are loaded by the threads.
-template <class R, int NTR, int TX, int TY, bool IMM, bool LEARNED = false, bool DECOMP = false, bool TMA = false>
-__global__ void __launch_bounds__(TX *TY, LEARNED ? PU_LEARNED_XY_MIN_BLOCKS : (sizeof(R) == 4 ? PU_XY_MIN_BLOCKS : 512 / (TX * TY))) k_xy(const Grid<R> G, const R *__restrict__ sin, R *__restrict__ txy, const __grid_constant__ XyMaps maps) {
+// SPLIT: threads per cell.
+template <class R, int NTR, int TX, int TY, bool IMM, bool LEARNED = false, bool DECOMP = false, bool TMA = false,
+          int SPLIT = 1>
+__global__ void __launch_bounds__(TX *TY *SPLIT, SPLIT > 1 ? 1024 / (TX * TY * SPLIT) : LEARNED ? PU_LEARNED_XY_MIN_BLOCKS : (sizeof(R) == 4 ? PU_XY_MIN_BLOCKS : 512 / (TX * TY))) k_xy(const Grid<R> G, const R *__restrict__ sin, R *__restrict__ txy, const __grid_constant__ XyMaps maps) {
   using Sh = XYShape<R, NTR, TX, TY, IMM, LEARNED>;
-  constexpr int F = Sh::F, S = Sh::S, NT = Sh::NT, HX = Sh::HX, HY = Sh::HY, EN = Sh::EN, FN = Sh::FN;
+  constexpr int F = Sh::F, S = Sh::S, NT = Sh::NT * SPLIT, HX = Sh::HX, HY = Sh::HY, EN = Sh::EN, FN = Sh::FN;
+  static_assert(SPLIT == 1 || (sizeof(R) == 4 && !LEARNED), "split positions: the packed limiter");
   static_assert(!TMA || (Sh::TMA_FITS && !DECOMP && !IMM), "TMA staging: 16x16 FP32 tiles, plain domains");
   extern __shared__ __align__(16) unsigned char smem_xy[];
   unsigned char *smem_raw = TMA ? smem_xy + ((128u - (tma::saddr(smem_xy) & 127u)) & 127u) : smem_xy;
@@ -766,7 +783,7 @@ __global__ void __launch_bounds__(TX *TY, LEARNED ? PU_LEARNED_XY_MIN_BLOCKS : (
   if constexpr ((!std::is_same<R, float>::value || PU_PACKED_LIMITER) && !LEARNED) {
     packed = G.weno_all != 0;
     if (packed) {
-      recon_inner<R, NT, F, TY, TX, false>([](int, int) { return true; }, mask_xc, vals_xc, store_xc);
+      recon_inner<R, NT, SPLIT, F, TY, TX, false>([](int, int) { return true; }, mask_xc, vals_xc, store_xc);
       // Halo pairs of the x lines, and already those of the y lines (kept in
       // YO until the y phase), so that every thread takes one pair here and
       // the y phase is the inner rounds alone.
@@ -830,7 +847,7 @@ __global__ void __launch_bounds__(TX *TY, LEARNED ? PU_LEARNED_XY_MIN_BLOCKS : (
   __syncthreads();
 
   // 4. x divergence of this thread's cell.
-  const int r = tid / TX, c = tid % TX;
+  const int cell = SPLIT == 1 ? tid : tid % (TX * TY), r = cell / TX, c = cell % TX;
   R tend[S];
 #pragma unroll
   for (int s = 0; s < S; s++) tend[s] = -(FL[s * FN + r * (TX + 1) + c + 1] - FL[s * FN + r * (TX + 1) + c]) * G.rdx;
@@ -850,7 +867,7 @@ __global__ void __launch_bounds__(TX *TY, LEARNED ? PU_LEARNED_XY_MIN_BLOCKS : (
       __syncthreads();   // step 4 has read the flux buffer that holds the queue
       n_fb += recon_learned<NT>(G, sW, queue, qn + 1, F * Sh::EYN, load_y, store_y);
     } else if (packed) {
-      recon_inner<R, NT, F, TX, TY, true>([](int, int) { return true; }, mask_yc, vals_yc, [&](int f, int cc, int rr, R qL, R qR) {
+      recon_inner<R, NT, SPLIT, F, TX, TY, true>([](int, int) { return true; }, mask_yc, vals_yc, [&](int f, int cc, int rr, R qL, R qR) {
         EL[f * EN + rr * TX + cc] = qL;
         ER[f * EN + rr * TX + cc] = qR;
       });
@@ -906,7 +923,7 @@ __global__ void __launch_bounds__(TX *TY, LEARNED ? PU_LEARNED_XY_MIN_BLOCKS : (
   }
 
   const int gi = i0 + c, gj = j0 + r;
-  if (gi < nx && gj < ny) {
+  if (gi < nx && gj < ny && (SPLIT == 1 || tid < TX * TY)) {
     const size_t idx = plane + size_t(gj) * nx + gi;
 #pragma unroll
     for (int s = 0; s < S; s++) txy[s * G.N + idx] = tend[s];
@@ -1325,13 +1342,15 @@ struct ZtMaps {
 // fit, the cell inputs are read per thread as without it.  Columns beyond
 // the domain read zero there instead of the last column; their results are
 // discarded either way.
-template <class R, int NTR, int TX, int TZ, bool IMM, bool TMA = false>
-__global__ void __launch_bounds__(TX *TZ, sizeof(R) == 4 ? PU_ZT_MIN_BLOCKS : PU_ZT_MIN_BLOCKS_F64)
+// SPLIT: threads per cell.
+template <class R, int NTR, int TX, int TZ, bool IMM, bool TMA = false, int SPLIT = 1>
+__global__ void __launch_bounds__(TX *TZ *SPLIT,
+                                  SPLIT > 1 ? 1 : sizeof(R) == 4 ? PU_ZT_MIN_BLOCKS : PU_ZT_MIN_BLOCKS_F64)
     k_zt(const Grid<R> G, const R *__restrict__ sin, const R *sn, R *sout, const R *__restrict__ txy, R a_n, R a_dt,
          int n_enforce, const __grid_constant__ ZtMaps maps) {
   static_assert(!TMA || sizeof(R) == 4, "TMA staging: FP32");
   using Sh = ZTShape<R, NTR, TX, TZ, IMM>;
-  constexpr int F = Sh::F, S = Sh::S, NT = Sh::NT, HZ = Sh::HZ;
+  constexpr int F = Sh::F, S = Sh::S, NT = Sh::NT * SPLIT, HZ = Sh::HZ;
   extern __shared__ __align__(16) unsigned char smem_zt[];
   unsigned char *smem_raw = TMA ? smem_zt + ((128u - (tma::saddr(smem_zt) & 127u)) & 127u) : smem_zt;
   R *H = reinterpret_cast<R *>(smem_raw);   // [F][HZ][TX]
@@ -1464,7 +1483,7 @@ __global__ void __launch_bounds__(TX *TZ, sizeof(R) == 4 ? PU_ZT_MIN_BLOCKS : PU
   };
   // Cells up to nz - 1, and cell nz in periodic z (face nz reads it).
   const int top = wall ? nz - 1 : nz;
-  recon_inner<R, NT, F, TX, TZ, true>([&](int, int q) { return k0 - 1 + q <= top; }, mask, vals, [&](int f, int c, int q, R qL, R qR) {
+  recon_inner<R, NT, SPLIT, F, TX, TZ, true>([&](int, int q) { return k0 - 1 + q <= top; }, mask, vals, [&](int f, int c, int q, R qL, R qR) {
     EL[(f * (TZ + 2) + q) * TX + c] = qL;
     ER[(f * (TZ + 2) + q) * TX + c] = qR;
   });
@@ -1490,7 +1509,7 @@ __global__ void __launch_bounds__(TX *TZ, sizeof(R) == 4 ? PU_ZT_MIN_BLOCKS : PU
   // barrier -- then the divergence, sources, stage combination and
   // enforcement of the cell.
   const int c = tid % TX, kz = tid / TX, k = k0 + kz, gi = i0 + c;
-  if (gi >= nx || k >= nz) return;
+  if (gi >= nx || k >= nz || kz >= TZ) return;
   auto face_flux = [&](int fz, R (&fl)[S]) {
     const int cf = k0 + fz;
     R Lf[F], Rf[F];

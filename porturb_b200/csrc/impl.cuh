@@ -748,6 +748,21 @@ struct Impl : ImplBase {
     return configure();
   }
 
+  // Whether the stage kernels take PU_SMALL_SPLIT threads per cell: with that
+  // many, the x/y and the z launch both fit the 148 SMs at once, 1024 threads
+  // each (64 registers a thread).  Both or none: such a z block fills an SM and
+  // cannot start beside a last wave of ordinary x/y blocks.  Measured, us per
+  // step, one thread per cell / four: 32x32x32 74 / 54, 64x4x32 46 / 33,
+  // 32x29x31 79 / 66, 24x24x24 54 / 53; with the z kernel alone split,
+  // 33x29x31 86 / 136.
+  bool split_small() const {
+    const size_t nxy = small_tile ? size_t(blocks(cfg.nx, XTX_SM)) * blocks(cfg.ny, XTY_SM) * (XTX_SM * XTY_SM)
+                                  : size_t(blocks(cfg.nx, XTX_BIG)) * blocks(cfg.ny, XTY_BIG) * (XTX_BIG * XTY_BIG);
+    const size_t nzt = size_t(blocks(cfg.nx, ZT_X)) * cfg.ny * blocks(cfg.nz, ZT_Z) * (ZT_X * ZT_Z);
+    return std::is_same<R, float>::value && z_tiled(learned_active()) && !dc.on &&
+           std::max(nxy * cfg.nz, nzt) * PU_SMALL_SPLIT <= size_t(148) * 1024;
+  }
+
   template <int X, int Z>
   int zt_configure() {
     PU_CK(cudaFuncSetAttribute(k_zt<R, NTR, X, Z, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -759,6 +774,29 @@ struct Impl : ImplBase {
                                  int(ZTShape<R, NTR, X, Z, false>::tma_bytes)));
       PU_CK(cudaFuncSetAttribute(k_zt<R, NTR, X, Z, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  int(ZTShape<R, NTR, X, Z, true>::tma_bytes)));
+    }
+    return PU_OK;
+  }
+
+  // The forms with PU_SMALL_SPLIT threads per cell.
+  int split_configure() {
+    if constexpr (std::is_same<R, float>::value) {
+      constexpr int SP = PU_SMALL_SPLIT;
+      auto set = [](const void *k, size_t bytes) {
+        return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes));
+      };
+      PU_CK(set((const void *)k_zt<R, NTR, ZT_X, ZT_Z, false, false, SP>, ZTShape<R, NTR, ZT_X, ZT_Z, false>::bytes));
+      PU_CK(set((const void *)k_zt<R, NTR, ZT_X, ZT_Z, true, false, SP>, ZTShape<R, NTR, ZT_X, ZT_Z, true>::bytes));
+      PU_CK(set((const void *)k_zt<R, NTR, ZT_X, ZT_Z, false, true, SP>, ZTShape<R, NTR, ZT_X, ZT_Z, false>::tma_bytes));
+      PU_CK(set((const void *)k_zt<R, NTR, ZT_X, ZT_Z, true, true, SP>, ZTShape<R, NTR, ZT_X, ZT_Z, true>::tma_bytes));
+      PU_CK(set((const void *)k_xy<R, NTR, XTX_BIG, XTY_BIG, false, false, false, false, SP>,
+                XYShape<R, NTR, XTX_BIG, XTY_BIG, false>::bytes));
+      PU_CK(set((const void *)k_xy<R, NTR, XTX_BIG, XTY_BIG, true, false, false, false, SP>,
+                XYShape<R, NTR, XTX_BIG, XTY_BIG, true>::bytes));
+      PU_CK(set((const void *)k_xy<R, NTR, XTX_SM, XTY_SM, false, false, false, false, SP>,
+                XYShape<R, NTR, XTX_SM, XTY_SM, false>::bytes));
+      PU_CK(set((const void *)k_xy<R, NTR, XTX_SM, XTY_SM, true, false, false, false, SP>,
+                XYShape<R, NTR, XTX_SM, XTY_SM, true>::bytes));
     }
     return PU_OK;
   }
@@ -791,6 +829,7 @@ struct Impl : ImplBase {
     PU_CK(cudaFuncSetAttribute(k_z<R, NTR, ZTX, ZTY, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                int(ZShape<R, NTR, ZTX, ZTY>::bytes)));
     PU_TRY((zt_configure<ZT_X, ZT_Z>()));
+    PU_TRY(split_configure());
     if constexpr (std::is_same<R, float>::value) {
       PU_TRY((zt_configure<16, 16>()));
       PU_TRY((zt_configure<32, 8>()));
@@ -1119,6 +1158,18 @@ struct Impl : ImplBase {
     Grid<R> Gt = G;
     Gt.i_first = tx0 * XTX_BIG;
     Gt.j_first = ty0 * XTY_BIG;
+    if constexpr (std::is_same<R, float>::value && !DEC) {
+      if (split_small()) {
+        constexpr int SP = PU_SMALL_SPLIT;
+        Grid<R> Gs = Gt;
+        Gs.k_first = k0;
+        // One launch: a few levels more of immersed code cost less than a second one.
+        xy_launch(k_xy<R, NTR, XTX_BIG, XTY_BIG, IMM, false, false, false, SP>, true, dim3(bx, by, k1 - k0), Sh::NT * SP,
+                  Sh::bytes, Gs, sin, t, xy_maps[b]);
+        PU_LAUNCHED();
+        return PU_OK;
+      }
+    }
     if (kl > k0) {
       Grid<R> Gi = Gt;
       Gi.k_first = k0;
@@ -1170,7 +1221,21 @@ struct Impl : ImplBase {
     const dim3 g(blocks(cfg.nx, X), unsigned(cfg.ny), unsigned(c1 - c0));
     bool staged = false;
     if constexpr (std::is_same<R, float>::value) {
-      if (zt_tma && static_cast<const void *>(sin) == s[b]) {
+      const bool tma = zt_tma && static_cast<const void *>(sin) == s[b];
+      if constexpr (Z == ZT_Z) {
+        if (split_small()) {
+          constexpr int SP = PU_SMALL_SPLIT;
+          if (tma)
+            launch_early(k_zt<R, NTR, X, Z, IMM, true, SP>, g, X * Z * SP, Zs::tma_bytes, st, Gc, sin, sn, sout, t, a_n,
+                         a_dt, n_enforce, maps);
+          else
+            launch_early(k_zt<R, NTR, X, Z, IMM, false, SP>, g, X * Z * SP, Zs::bytes, st, Gc, sin, sn, sout, t, a_n,
+                         a_dt, n_enforce, maps);
+          PU_LAUNCHED();
+          return PU_OK;
+        }
+      }
+      if (tma) {
         launch_early(k_zt<R, NTR, X, Z, IMM, true>, g, X * Z, Zs::tma_bytes, st, Gc, sin, sn, sout, t, a_n, a_dt,
                      n_enforce, maps);
         staged = true;
@@ -1209,7 +1274,14 @@ struct Impl : ImplBase {
     if (small_tile) {
       using Sh = XYShape<R, NTR, XTX_SM, XTY_SM, IMM, L>;
       dim3 g(blocks(cfg.nx, XTX_SM), blocks(cfg.ny, XTY_SM), cfg.nz);
-      xy_launch(k_xy<R, NTR, XTX_SM, XTY_SM, IMM, L, DEC>, !DEC, g, Sh::NT, Sh::bytes, G, sin, t, xy_maps[b]);
+      bool split = false;
+      if constexpr (std::is_same<R, float>::value && !DEC && !L) {
+        split = split_small();
+        if (split)
+          xy_launch(k_xy<R, NTR, XTX_SM, XTY_SM, IMM, false, false, false, PU_SMALL_SPLIT>, true, g,
+                    Sh::NT * PU_SMALL_SPLIT, Sh::bytes, G, sin, t, xy_maps[b]);
+      }
+      if (!split) xy_launch(k_xy<R, NTR, XTX_SM, XTY_SM, IMM, L, DEC>, !DEC, g, Sh::NT, Sh::bytes, G, sin, t, xy_maps[b]);
       PU_LAUNCHED();
     } else if (L) {
       using Sh = XYShape<R, NTR, LTX, LTY, IMM, L>;

@@ -58,3 +58,30 @@ def test_tiled_z_kernel_in_fp64(name, gpu_lib):
     st_m, tr_m, _ = gpu_run(case, "f64", 4, dt, z_chunk=16)
     for a, b in list(zip(st_t, st_m)) + list(zip(tr_t, tr_m)):
         assert np.abs(a - b).max() <= 1e-12 * max(np.abs(b).max(), 1e-300)
+
+
+LARGE = {
+    "immersed": lambda: cases.small_mixed(nx=72, ny=40, nz=40),
+    "three_tracers_partial": lambda: cases.small_mixed(nx=70, ny=41, nz=45, ntr=3, immersed=False),
+    "periodic_z": lambda: cases.small_mixed(nx=64, ny=48, nz=70, bc_z="periodic", immersed=False),
+    "thin": lambda: cases.small_mixed(nx=160, ny=5, nz=64),
+}
+
+
+@pytest.mark.parametrize("name", sorted(LARGE))
+def test_one_thread_per_cell(name, gpu_lib):
+    """Grids of more blocks than fit the SMs at four threads per cell, which the
+    grids above all take: the tile gives the march's bits there too, with the
+    x/y kernel's tiles staged through TMA or loaded by its threads."""
+    case = LARGE[name]()
+    _, _, g = gpu_run(case, "f32", 0, 0.0)
+    dt = 0.9 * g.compute_time_step()
+    st_t, tr_t, _ = gpu_run(case, "f32", 2, dt)
+    for kw in (dict(z_chunk=16), dict(thread_loads=True)):
+        st_m, tr_m, _ = gpu_run(case, "f32", 2, dt, **kw)
+        assert np.array_equal(st_t, st_m) and np.array_equal(tr_t, tr_m), kw
+    # A case of one such tile column more or less: four threads per cell.
+    block = case.block(0, 0, 16, min(case.ny, 16))
+    st_s, tr_s, _ = gpu_run(block, "f32", 2, dt)
+    st_c, tr_c, _ = gpu_run(block, "f32", 2, dt, z_chunk=16)
+    assert np.array_equal(st_s, st_c) and np.array_equal(tr_s, tr_c)
