@@ -334,10 +334,10 @@ struct XYShape {
   // stencil masks of the x lines ([TY][TX+2]) and the y lines ([TY+2][TX]).
   static constexpr size_t MB = (size_t(HY) * HX + 15) / 16 * 16;
   static constexpr size_t MASKB = (size_t(2) * (TY * (TX + 2) + (TY + 2) * TX) + 15) / 16 * 16;
-  // Learned mode: per-warp network scratch and two fallback counters; the
+  // Learned mode: the network's fragments, per-warp scratch and two counters; the
   // fallback queue (16-bit stencil indices) lives in the flux buffer, which
   // is idle while edges are reconstructed.
-  static constexpr size_t learned_bytes = LEARNED ? size_t(NT / 32) * mlp::WARP_SMEM_BYTES + 16 : 0;
+  static constexpr size_t learned_bytes = LEARNED ? size_t(NT / 32) * mlp::WARP_SMEM_BYTES + mlp::FRAG_BYTES + 16 : 0;
   static constexpr size_t layout_bytes = sizeof(R) * (size_t(F) * HY * HX + 2 * size_t(F) * EN + size_t(S) * FN + YON) +
                                          (IMM ? MB + MASKB : 0) + learned_bytes;
   static constexpr size_t bytes = layout_bytes;
@@ -387,8 +387,8 @@ struct XyMaps {
 // entry (learned in the low half, fallbacks in the high half).  Returns the
 // number of fallbacks.
 template <int NT, class Load, class Store>
-__device__ __forceinline__ int recon_learned(const Grid<float> &G, uint32_t *sW, uint16_t *queue, int *qn, int total,
-                                             Load load, Store store) {
+__device__ __forceinline__ int recon_learned(const Grid<float> &G, const uint4 *sF, uint32_t *sW, uint16_t *queue,
+                                             int *qn, int total, Load load, Store store) {
   const int tid = threadIdx.x, lane = tid & 31;
   const unsigned below = (1u << lane) - 1u;
   for (int base = tid & ~31; base < total; base += NT) {
@@ -409,23 +409,22 @@ __device__ __forceinline__ int recon_learned(const Grid<float> &G, uint32_t *sW,
   }
   __syncthreads();
   const int nl = *qn & 0xffff, nf = *qn >> 16;
-  if ((tid & ~31) < nl) {
-    MlpLane L;
-    load_lane(G.ml_frags, L);
-    for (int base = tid & ~31; base < nl; base += NT) {
-      const bool valid = base + lane < nl;
-      const int it = queue[valid ? base + lane : base];
-      float s[9], x[9], wl[5], wr[5];
-      unsigned imm;
-      bool any10;
-      load(it, s, imm, any10);
+  for (int base = tid & ~31; base < nl; base += NT) {
+    const bool valid = base + lane < nl;
+    const int it = queue[valid ? base + lane : base];
+    float s[9], wl[5], wr[5];
+    unsigned imm;
+    bool any10;
+    load(it, s, imm, any10);
+    {
+      float x[9];
       normalize9(s, x);
-      mlp_warp_weights(L, sW, x, wl, wr);
-      if (valid) {
-        float qL, qR;
-        edges_from_weights(s, wl, wr, qL, qR);
-        store(it, qL, qR);
-      }
+      mlp_warp_weights(sF, sW, x, wl, wr);
+    }
+    if (valid) {
+      float qL, qR;
+      edges_from_weights(s, wl, wr, qL, qR);
+      store(it, qL, qR);
     }
   }
   const int half = (nf + 1) / 2;
@@ -595,7 +594,8 @@ __global__ void __launch_bounds__(TX *TY *SPLIT, SPLIT > 1 ? 1024 / (TX * TY * S
   uint16_t *MY = MX + TY * (TX + 2);                          // [TY+2][TX] y-stencil masks
   unsigned char *lrn = reinterpret_cast<unsigned char *>(YO + Sh::YON) + (IMM ? Sh::MB + Sh::MASKB : 0);
   int *qn = reinterpret_cast<int *>(lrn);                    // [2] fallback counts (x, y)
-  uint32_t *sW = reinterpret_cast<uint32_t *>(lrn + 16) + (threadIdx.x >> 5) * (mlp::WARP_SMEM_BYTES / 4);
+  uint4 *sF = reinterpret_cast<uint4 *>(lrn + 16);           // the network's fragments
+  uint32_t *sW = reinterpret_cast<uint32_t *>(lrn + 16 + mlp::FRAG_BYTES) + (threadIdx.x >> 5) * (mlp::WARP_SMEM_BYTES / 4);
   uint16_t *queue = reinterpret_cast<uint16_t *>(FL);
 
   const int tid = threadIdx.x;
@@ -605,6 +605,7 @@ __global__ void __launch_bounds__(TX *TY *SPLIT, SPLIT > 1 ? 1024 / (TX * TY * S
   const size_t plane = size_t(k) * G.NP;
   const bool sim2d = G.sim2d != 0;
   if (LEARNED && tid < 2) qn[tid] = 0;
+  if constexpr (LEARNED) load_frags(G.ml_frags, sF, NT);
   if (!G.late) previous_done();
   next_kernel_may_start();
 
@@ -805,7 +806,7 @@ __global__ void __launch_bounds__(TX *TY *SPLIT, SPLIT > 1 ? 1024 / (TX * TY * S
     }
   }
   if constexpr (LEARNED) {
-    n_fb += recon_learned<NT>(G, sW, queue, qn, F * Sh::EXN, load_x, store_x);
+    n_fb += recon_learned<NT>(G, sF, sW, queue, qn, F * Sh::EXN, load_x, store_x);
   } else if (!packed) {
     for (int it = tid; it < F * Sh::EXN; it += NT) {
       R s[9];
@@ -865,7 +866,7 @@ __global__ void __launch_bounds__(TX *TY *SPLIT, SPLIT > 1 ? 1024 / (TX * TY * S
     };
     if constexpr (LEARNED) {
       __syncthreads();   // step 4 has read the flux buffer that holds the queue
-      n_fb += recon_learned<NT>(G, sW, queue, qn + 1, F * Sh::EYN, load_y, store_y);
+      n_fb += recon_learned<NT>(G, sF, sW, queue, qn + 1, F * Sh::EYN, load_y, store_y);
     } else if (packed) {
       recon_inner<R, NT, SPLIT, F, TX, TY, true>([](int, int) { return true; }, mask_yc, vals_yc, [&](int f, int cc, int rr, R qL, R qR) {
         EL[f * EN + rr * TX + cc] = qL;
@@ -958,7 +959,8 @@ struct ZShape {
   // edges of the current and the previous cell; all thread-private columns.
   // Learned mode adds per-warp network scratch and a per-warp fallback queue
   // of up to F*32 entries.
-  static constexpr size_t learned_bytes = LEARNED ? size_t(NT / 32) * (mlp::WARP_SMEM_BYTES + F * 32 * 4) : 0;
+  static constexpr size_t learned_bytes =
+      LEARNED ? size_t(NT / 32) * (mlp::WARP_SMEM_BYTES + F * 32 * 4) + mlp::FRAG_BYTES : 0;
   static constexpr size_t bytes = sizeof(R) * (9 + 3) * size_t(F) * NT + learned_bytes;
 };
 
@@ -1027,12 +1029,17 @@ __global__ void __launch_bounds__(TX *TY, LEARNED ? PU_LEARNED_Z_MIN_BLOCKS : (s
   R *ring = reinterpret_cast<R *>(smem_raw);   // [9][F][NT]
   R *eL = ring + 9 * F * NT;                     // [F][NT]
   R *eR = eL + F * NT;                           // [2][F][NT]
-  uint32_t *sW = reinterpret_cast<uint32_t *>(eR + 2 * F * NT) +
+  uint4 *sF = reinterpret_cast<uint4 *>(eR + 2 * F * NT);   // the network's fragments
+  uint32_t *sW = reinterpret_cast<uint32_t *>(eR + 2 * F * NT) + mlp::FRAG_BYTES / 4 +
                  (threadIdx.x >> 5) * ((mlp::WARP_SMEM_BYTES + F * 32 * 4) / 4);
   uint32_t *wq = sW + mlp::WARP_SMEM_BYTES / 4;  // per-warp fallback queue
   unsigned long long n_learned = 0, n_fallback = 0;
   const int tid = threadIdx.x;
   const int i = blockIdx.x * TX + tid % TX, j = blockIdx.y * TY + tid / TX;
+  if constexpr (LEARNED) {   // every block is full
+    load_frags(G.ml_frags, sF, NT);
+    __syncthreads();
+  }
   if (i >= G.nx || j >= G.ny) return;            // no block-wide synchronisation below
   const int nz = G.nz;
   const int k0 = blockIdx.z * kchunk, k1 = min(nz, k0 + kchunk);
@@ -1152,22 +1159,18 @@ __global__ void __launch_bounds__(TX *TY, LEARNED ? PU_LEARNED_Z_MIN_BLOCKS : (s
           eL[o] = qL;
           eR[par * F * NT + o] = qR;
         };
-        if (nl) {
-          MlpLane L;
-          load_lane(G.ml_frags, L);
 #pragma unroll 1
-          for (int base = 0; base < nl; base += 32) {
-            const bool valid = base + lane < nl;
-            const unsigned e = wq[valid ? base + lane : base];
-            float s[9], x[9], wl[5], wr[5];
-            load_q(e, s);
-            normalize9(s, x);
-            mlp_warp_weights(L, sW, x, wl, wr);
-            if (valid) {
-              float qL, qR;
-              edges_from_weights(s, wl, wr, qL, qR);
-              store_q(e, qL, qR);
-            }
+        for (int base = 0; base < nl; base += 32) {
+          const bool valid = base + lane < nl;
+          const unsigned e = wq[valid ? base + lane : base];
+          float s[9], x[9], wl[5], wr[5];
+          load_q(e, s);
+          normalize9(s, x);
+          mlp_warp_weights(sF, sW, x, wl, wr);
+          if (valid) {
+            float qL, qR;
+            edges_from_weights(s, wl, wr, qL, qR);
+            store_q(e, qL, qR);
           }
         }
         const int half = (cnt + 1) / 2;

@@ -372,7 +372,8 @@ struct ImplBase {
     cudaMemcpyAsync(dx, x, size_t(n) * 9 * sizeof(float), cudaMemcpyHostToDevice, st);
     if (use_mma) {
       const int warps = 4;
-      k_mlp_eval_mma<<<unsigned((n + 32 * warps - 1) / (32 * warps)), 32 * warps, warps * mlp::WARP_SMEM_BYTES, st>>>(
+      k_mlp_eval_mma<<<unsigned((n + 32 * warps - 1) / (32 * warps)), 32 * warps,
+                       mlp::FRAG_BYTES + warps * mlp::WARP_SMEM_BYTES, st>>>(
           ml_frags, dx, n, dl, dr);
     } else {
       k_mlp_eval<<<unsigned((n + 255) / 256), 256, 0, st>>>(ml_wq, dx, n, dl);

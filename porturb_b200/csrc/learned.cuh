@@ -447,14 +447,15 @@ static __global__ void __launch_bounds__(128) k_mlp_eval_mma(const uint32_t *__r
                                                       long n, float *__restrict__ wl_out, float *__restrict__ wr_out) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  uint32_t *sW = reinterpret_cast<uint32_t *>(smem_raw + warp * mlp::WARP_SMEM_BYTES);
-  MlpLane L;
-  load_lane(frags, L);
+  uint4 *sF = reinterpret_cast<uint4 *>(smem_raw);
+  uint32_t *sW = reinterpret_cast<uint32_t *>(smem_raw + mlp::FRAG_BYTES + warp * mlp::WARP_SMEM_BYTES);
+  load_frags(frags, sF, blockDim.x);
+  __syncthreads();
   const long q = (long(blockIdx.x) * (blockDim.x >> 5) + warp) * 32 + lane;
   float x[9], wl[5], wr[5];
 #pragma unroll
   for (int m = 0; m < 9; m++) x[m] = q < n ? xs[q * 9 + m] : 0.f;
-  mlp_warp_weights(L, sW, x, wl, wr);
+  mlp_warp_weights(sF, sW, x, wl, wr);
   if (q < n) {
 #pragma unroll
     for (int k = 0; k < 5; k++) {

@@ -29,7 +29,10 @@ constexpr int OFF_B2 = OFF_W2 + NH * NH;
 constexpr int OFF_W3 = OFF_B2 + NH;
 constexpr int OFF_B3 = OFF_W3 + NOUT * NH;
 constexpr int NPARAM = OFF_B3 + NOUT;   // 1541
-constexpr int FRAG_WORDS = 38;          // per lane: 28 bf16x2 operand words + 10 FP32 bias values
+// Operand fragments of the network, in shared memory while a kernel runs: ten
+// groups of 16 bytes per lane (28 bf16x2 operand words, 10 FP32 biases, 2
+// unused words), group by group over the 32 lanes.
+constexpr int FRAG_GROUPS = 10, FRAG_WORDS = 4 * FRAG_GROUPS;
 constexpr int FRAG_BYTES = 32 * FRAG_WORDS * 4;
 // Per-warp shared memory: 64 input rows of 16 bf16 (2 KB), then the logits
 // column by column with a 68-float stride (5 x 68 floats), bank-conflict
@@ -79,8 +82,9 @@ __device__ __forceinline__ uint32_t bf16_bits(float x) {
 }
 
 // Per-lane operand fragments of mma.m16n8k16 (B is K x N, K = layer input,
-// N = layer output), word layout: w1[4][2], w2[2][4][2], w3[2][2] (bfloat16
-// pairs, lower k in the low half), then b2[4][2], b3[2] as FP32 bits.
+// N = layer output; bfloat16 pairs, lower k in the low half).  Groups of four
+// words: 0-1 W1's four output tiles, 2-5 W2's output tiles (both K halves of
+// each), 6 W3, 7-8 b2, 9 b3 (FP32 bits).
 static __global__ void k_mlp_frags(const float *__restrict__ theta, uint32_t *__restrict__ frags) {
   using namespace mlp;
   const int lane = threadIdx.x;
@@ -96,70 +100,46 @@ static __global__ void k_mlp_frags(const float *__restrict__ theta, uint32_t *__
   auto W2 = [&](int o, int i) { return theta[OFF_W2 + o * NH + i]; };
   auto W3 = [&](int o, int i) { return o < NOUT ? theta[OFF_W3 + o * NH + i] : 0.f; };
   auto pk = [](float lo, float hi) { return bf16_bits(lo) | (bf16_bits(hi) << 16); };
-  uint32_t *f = frags + lane * FRAG_WORDS;
   int w = 0;
+  auto put = [&](uint32_t v) {
+    frags[((w >> 2) * 32 + lane) * 4 + (w & 3)] = v;
+    w++;
+  };
   for (int n = 0; n < 4; n++) {
-    f[w++] = pk(W1(8 * n + g, 2 * t), W1(8 * n + g, 2 * t + 1));
-    f[w++] = pk(W1(8 * n + g, 2 * t + 8), W1(8 * n + g, 2 * t + 9));
+    put(pk(W1(8 * n + g, 2 * t), W1(8 * n + g, 2 * t + 1)));
+    put(pk(W1(8 * n + g, 2 * t + 8), W1(8 * n + g, 2 * t + 9)));
   }
-  for (int s = 0; s < 2; s++)
-    for (int n = 0; n < 4; n++) {
-      f[w++] = pk(W2(8 * n + g, 16 * s + 2 * t), W2(8 * n + g, 16 * s + 2 * t + 1));
-      f[w++] = pk(W2(8 * n + g, 16 * s + 2 * t + 8), W2(8 * n + g, 16 * s + 2 * t + 9));
+  for (int n = 0; n < 4; n++)
+    for (int s = 0; s < 2; s++) {
+      put(pk(W2(8 * n + g, 16 * s + 2 * t), W2(8 * n + g, 16 * s + 2 * t + 1)));
+      put(pk(W2(8 * n + g, 16 * s + 2 * t + 8), W2(8 * n + g, 16 * s + 2 * t + 9)));
     }
   for (int s = 0; s < 2; s++) {
-    f[w++] = pk(W3(g, 16 * s + 2 * t), W3(g, 16 * s + 2 * t + 1));
-    f[w++] = pk(W3(g, 16 * s + 2 * t + 8), W3(g, 16 * s + 2 * t + 9));
+    put(pk(W3(g, 16 * s + 2 * t), W3(g, 16 * s + 2 * t + 1)));
+    put(pk(W3(g, 16 * s + 2 * t + 8), W3(g, 16 * s + 2 * t + 9)));
   }
   for (int n = 0; n < 4; n++) {
-    f[w++] = __float_as_uint(theta[OFF_B2 + 8 * n + 2 * t]);
-    f[w++] = __float_as_uint(theta[OFF_B2 + 8 * n + 2 * t + 1]);
+    put(__float_as_uint(theta[OFF_B2 + 8 * n + 2 * t]));
+    put(__float_as_uint(theta[OFF_B2 + 8 * n + 2 * t + 1]));
   }
-  f[w++] = __float_as_uint(2 * t < NOUT ? theta[OFF_B3 + 2 * t] : 0.f);
-  f[w++] = __float_as_uint(2 * t + 1 < NOUT ? theta[OFF_B3 + 2 * t + 1] : 0.f);
+  put(__float_as_uint(2 * t < NOUT ? theta[OFF_B3 + 2 * t] : 0.f));
+  put(__float_as_uint(2 * t + 1 < NOUT ? theta[OFF_B3 + 2 * t + 1] : 0.f));
+  put(0u);
+  put(0u);
 }
 
-// One lane's operand fragments, held in registers for the life of a kernel.
-struct MlpLane {
-  uint32_t w1[4][2], w2[2][4][2], w3[2][2];
-  float b2[4][2], b3[2];
-};
-
-__device__ __forceinline__ void load_lane(const uint32_t *__restrict__ frags, MlpLane &L) {
-  const uint32_t *f = frags + (threadIdx.x & 31) * mlp::FRAG_WORDS;
-  int w = 0;
-#pragma unroll
-  for (int n = 0; n < 4; n++) {
-    L.w1[n][0] = __ldg(f + w++);
-    L.w1[n][1] = __ldg(f + w++);
-  }
-#pragma unroll
-  for (int s = 0; s < 2; s++)
-#pragma unroll
-    for (int n = 0; n < 4; n++) {
-      L.w2[s][n][0] = __ldg(f + w++);
-      L.w2[s][n][1] = __ldg(f + w++);
-    }
-#pragma unroll
-  for (int s = 0; s < 2; s++) {
-    L.w3[s][0] = __ldg(f + w++);
-    L.w3[s][1] = __ldg(f + w++);
-  }
-#pragma unroll
-  for (int n = 0; n < 4; n++) {
-    L.b2[n][0] = __uint_as_float(__ldg(f + w++));
-    L.b2[n][1] = __uint_as_float(__ldg(f + w++));
-  }
-  L.b3[0] = __uint_as_float(__ldg(f + w++));
-  L.b3[1] = __uint_as_float(__ldg(f + w++));
+// The fragments into shared memory, by the block's nt threads (the caller
+// synchronises).
+__device__ __forceinline__ void load_frags(const uint32_t *__restrict__ frags, uint4 *sF, int nt) {
+  for (int e = threadIdx.x; e < mlp::FRAG_GROUPS * 32; e += nt) sF[e] = __ldg(reinterpret_cast<const uint4 *>(frags) + e);
 }
 
-__device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], const uint32_t (&b)[2],
+__device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1,
                                          const float (&c)[4]) {
   asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
       "{%10,%11,%12,%13};\n"
       : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]), "f"(c[0]), "f"(c[1]), "f"(c[2]),
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(c[0]), "f"(c[1]), "f"(c[2]),
         "f"(c[3]));
 }
 
@@ -175,12 +155,12 @@ __device__ __forceinline__ uint32_t bf16x2(float lo, float hi) {
   return r;
 }
 
-// Input fragment k-step s of the next layer from output n-tiles 2s, 2s+1.
-__device__ __forceinline__ void acc_to_a(const float (&d)[4][4], int s, uint32_t (&a)[4]) {
-  a[0] = relu_bf16x2(d[2 * s][0], d[2 * s][1]);
-  a[1] = relu_bf16x2(d[2 * s][2], d[2 * s][3]);
-  a[2] = relu_bf16x2(d[2 * s + 1][0], d[2 * s + 1][1]);
-  a[3] = relu_bf16x2(d[2 * s + 1][2], d[2 * s + 1][3]);
+// Input fragment k-step s of the next layer from output tiles 2s (d0), 2s+1 (d1).
+__device__ __forceinline__ void acc_to_a(const float (&d0)[4], const float (&d1)[4], uint32_t (&a)[4]) {
+  a[0] = relu_bf16x2(d0[0], d0[1]);
+  a[1] = relu_bf16x2(d0[2], d0[3]);
+  a[2] = relu_bf16x2(d1[0], d1[1]);
+  a[3] = relu_bf16x2(d1[2], d1[3]);
 }
 
 // One warp evaluates the network on the 32 normalised stencils held by its
@@ -189,9 +169,15 @@ __device__ __forceinline__ void acc_to_a(const float (&d)[4][4], int s, uint32_t
 // the halves swapped when bit 2 of r is set, so the row stores and the
 // ldmatrix phases hit 8 distinct bank groups.  Returns each lane's left-edge
 // weights and the right-edge weights of its stencil.  All 32 lanes must call it.
+//
+// The four 16-row tiles go through each layer together: a tile's chain of
+// fourteen MMAs and the conversions between them is bound by their latency,
+// four of them interleave, and a layer's operands (sF) are read once per warp
+// call instead of staying in 38 registers (128x128x64 boundary layer: k_xy 640
+// -> 576 us, the z march 414 -> 398 us per launch).
 __device__ __forceinline__ int row_chunk(int r, int half) { return 2 * r + (half ^ ((r >> 2) & 1)); }
 
-__device__ __forceinline__ void mlp_warp_weights(const MlpLane &L, uint32_t *sW, const float (&x)[9], float (&wl)[5],
+__device__ __forceinline__ void mlp_warp_weights(const uint4 *sF, uint32_t *sW, const float (&x)[9], float (&wl)[5],
                                                  float (&wr)[5]) {
   using mlp::LOGIT_STRIDE;
   const int lane = threadIdx.x & 31;
@@ -206,48 +192,64 @@ __device__ __forceinline__ void mlp_warp_weights(const MlpLane &L, uint32_t *sW,
       make_uint4(bf16x2(x[8], x[7]), bf16x2(x[6], x[5]), bf16x2(x[4], x[3]), bf16x2(x[2], x[1]));
   rows[row_chunk(32 + lane, 1)] = make_uint4(bf16x2(x[0], 1.f), one, 0u, 0u);
   __syncwarp();
-#pragma unroll 1
-  for (int T = 0; T < 4; T++) {
-    uint32_t a[4];
-    const uint4 *src = rows + row_chunk(16 * T + (lane & 15), lane >> 4);
-    const unsigned addr = static_cast<unsigned>(__cvta_generic_to_shared(src));
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
-                 : "=r"(a[0]), "=r"(a[1]), "=r"(a[2]), "=r"(a[3])
-                 : "r"(addr)
-                 : "memory");
-    float d1[4][4];
+  const uint4 *F = sF + lane;
+  uint32_t a2[4][2][4], a3[4][2][4];
+  {
+    uint32_t a[4][4];
 #pragma unroll
-    for (int n = 0; n < 4; n++) {
-      const float c[4] = {0.f, 0.f, 0.f, 0.f};
-      mma_bf16(d1[n], a, L.w1[n], c);
+    for (int T = 0; T < 4; T++) {
+      const uint4 *src = rows + row_chunk(16 * T + (lane & 15), lane >> 4);
+      const unsigned addr = static_cast<unsigned>(__cvta_generic_to_shared(src));
+      asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+                   : "=r"(a[T][0]), "=r"(a[T][1]), "=r"(a[T][2]), "=r"(a[T][3])
+                   : "r"(addr)
+                   : "memory");
     }
-    uint32_t a2[2][4];
-    acc_to_a(d1, 0, a2[0]);
-    acc_to_a(d1, 1, a2[1]);
-    float d2[4][4];
+    const float zero[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-    for (int n = 0; n < 4; n++) {
-      const float c[4] = {L.b2[n][0], L.b2[n][1], L.b2[n][0], L.b2[n][1]};
-      mma_bf16(d2[n], a2[0], L.w2[0][n], c);
-      mma_bf16(d2[n], a2[1], L.w2[1][n], d2[n]);
+    for (int s = 0; s < 2; s++) {
+      const uint4 w = F[32 * s];
+#pragma unroll
+      for (int T = 0; T < 4; T++) {
+        float d0[4], d1[4];
+        mma_bf16(d0, a[T], w.x, w.y, zero);
+        mma_bf16(d1, a[T], w.z, w.w, zero);
+        acc_to_a(d0, d1, a2[T][s]);
+      }
     }
-    uint32_t a3[2][4];
-    acc_to_a(d2, 0, a3[0]);
-    acc_to_a(d2, 1, a3[1]);
-    float d3[4];
-    {
-      const float c[4] = {L.b3[0], L.b3[1], L.b3[0], L.b3[1]};
-      mma_bf16(d3, a3[0], L.w3[0], c);
-      mma_bf16(d3, a3[1], L.w3[1], d3);
+  }
+#pragma unroll
+  for (int s = 0; s < 2; s++) {
+    const uint4 w0 = F[32 * (2 + 2 * s)], w1 = F[32 * (3 + 2 * s)], b = F[32 * (7 + s)];
+    const float c0[4] = {__uint_as_float(b.x), __uint_as_float(b.y), __uint_as_float(b.x), __uint_as_float(b.y)};
+    const float c1[4] = {__uint_as_float(b.z), __uint_as_float(b.w), __uint_as_float(b.z), __uint_as_float(b.w)};
+#pragma unroll
+    for (int T = 0; T < 4; T++) {
+      float d0[4], d1[4];
+      mma_bf16(d0, a2[T][0], w0.x, w0.y, c0);
+      mma_bf16(d1, a2[T][0], w1.x, w1.y, c1);
+      mma_bf16(d0, a2[T][1], w0.z, w0.w, d0);
+      mma_bf16(d1, a2[T][1], w1.z, w1.w, d1);
+      acc_to_a(d0, d1, a3[T][s]);
     }
-    const int r0 = 16 * T + g, r1 = r0 + 8;
-    if (2 * t < 5) {
-      sZ[2 * t * LOGIT_STRIDE + r0] = d3[0];
-      sZ[2 * t * LOGIT_STRIDE + r1] = d3[2];
-    }
-    if (2 * t + 1 < 5) {
-      sZ[(2 * t + 1) * LOGIT_STRIDE + r0] = d3[1];
-      sZ[(2 * t + 1) * LOGIT_STRIDE + r1] = d3[3];
+  }
+  {
+    const uint4 w = F[32 * 6], b = F[32 * 9];
+    const float c[4] = {__uint_as_float(b.x), __uint_as_float(b.y), __uint_as_float(b.x), __uint_as_float(b.y)};
+#pragma unroll
+    for (int T = 0; T < 4; T++) {
+      float d3[4];
+      mma_bf16(d3, a3[T][0], w.x, w.y, c);
+      mma_bf16(d3, a3[T][1], w.z, w.w, d3);
+      const int r0 = 16 * T + g, r1 = r0 + 8;
+      if (2 * t < 5) {
+        sZ[2 * t * LOGIT_STRIDE + r0] = d3[0];
+        sZ[2 * t * LOGIT_STRIDE + r1] = d3[2];
+      }
+      if (2 * t + 1 < 5) {
+        sZ[(2 * t + 1) * LOGIT_STRIDE + r0] = d3[1];
+        sZ[(2 * t + 1) * LOGIT_STRIDE + r1] = d3[3];
+      }
     }
   }
   __syncwarp();
