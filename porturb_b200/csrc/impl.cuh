@@ -1263,6 +1263,26 @@ struct Impl : ImplBase {
     return zt_launch<false, X, Z>(G, sin, sn, sout, a_n, a_dt, n_enforce, b, ci, c1);
   }
 
+  // Levels per chunk of the learned z march, three of whose blocks fit an SM
+  // and all of which take about the time of their levels and 3 more (the two
+  // closing cells, the first planes): the chunk count that fills whole waves
+  // best.  128x128x64 columns in chunks of 16 levels are 512 blocks, 1.15
+  // waves: 398 us per launch, 332 us in three chunks; 64x64x48 195 and 118 us.
+  int learned_z_chunk() const {
+    const size_t cols = size_t(cfg.nx / ZTX) * (cfg.ny / ZTY);
+    int best = cfg.nz;
+    double cost = 1e300;
+    for (int c = 1; c <= (cfg.nz + 7) / 8; c++) {
+      const int kc = (cfg.nz + c - 1) / c;
+      const double t = double((cols * blocks(cfg.nz, kc) + 3 * 148 - 1) / (3 * 148)) * (kc + 3);
+      if (t < cost) {
+        cost = t;
+        best = kc;
+      }
+    }
+    return best;
+  }
+
   // One SSPRK3 stage: the x/y kernel (DEC: a decomposed tile reading its
   // received halo slabs), then the z march with the stage combination.
   template <bool IMM, bool LRN, bool DEC = false>
@@ -1302,7 +1322,9 @@ struct Impl : ImplBase {
       PU_TRY((xy_levels<IMM, DEC>(G, sin, b, 0, cfg.nz)));
     }
     prof_end(0, e0);
-    const int kc = cfg.z_chunk > 0 ? cfg.z_chunk : (cfg.nz < 16 ? cfg.nz : 16);
+    // The learned z march needs full warps: every block's columns inside the domain.
+    const bool lz = L && cfg.nx % ZTX == 0 && cfg.ny % ZTY == 0;
+    const int kc = cfg.z_chunk > 0 ? cfg.z_chunk : lz ? learned_z_chunk() : (cfg.nz < 16 ? cfg.nz : 16);
     dim3 gz(blocks(cfg.nx, ZTX), blocks(cfg.ny, ZTY), blocks(cfg.nz, kc));
     cudaEvent_t e1 = prof_begin();
     if (z_tiled(L)) {
@@ -1310,8 +1332,7 @@ struct Impl : ImplBase {
       prof_end(1, e1);
       return PU_OK;
     }
-    // The learned z march needs full warps: every block's columns inside the domain.
-    if (L && cfg.nx % ZTX == 0 && cfg.ny % ZTY == 0)
+    if (lz)
       k_z<R, NTR, ZTX, ZTY, IMM, L><<<gz, ZTX * ZTY, ZShape<R, NTR, ZTX, ZTY, L>::bytes, st>>>(
           G, sin, sn, sout, t, a_n, a_dt, n_enforce, kc);
     else
