@@ -172,6 +172,8 @@ __device__ __forceinline__ R pow1pm1(const Grid<R> &G, R x) {
 // until the kernel before has completed and its writes are visible (returns at
 // once in a kernel launched the ordinary way).  Every block calls it before it
 // ends, so a kernel that has completed implies that all before it have.
+// What the kernel before writes is read through plain pointers (no
+// __restrict__, no __ldg): a read-only load could be moved ahead of the wait.
 //   k_xy  waits first, then lets the z kernel start.  A second k_xy launch of
 //         the same stage (the plain levels after the immersed ones) reads and
 //         writes nothing of the first and waits only at its end (Grid::late):
@@ -214,16 +216,16 @@ __device__ __forceinline__ void prims_of(const Grid<R> &G, const R (&q)[5 + NTR]
 // The same from a state whose S fields lie N elements apart (the resident
 // arrays, N = nz*ny*nx, or a halo slab).
 template <class R, int NTR>
-__device__ __forceinline__ void prims_s(const Grid<R> &G, const R *__restrict__ s, size_t N, size_t idx, int k,
+__device__ __forceinline__ void prims_s(const Grid<R> &G, const R *s, size_t N, size_t idx, int k,
                                         R (&w)[6 + NTR]) {
   R q[5 + NTR];
 #pragma unroll
-  for (int v = 0; v < 5 + NTR; v++) q[v] = __ldg(s + v * N + idx);
+  for (int v = 0; v < 5 + NTR; v++) q[v] = s[v * N + idx];
   prims_of<R, NTR>(G, q, k, w);
 }
 
 template <class R, int NTR>
-__device__ __forceinline__ void prims(const Grid<R> &G, const R *__restrict__ s, size_t idx, int k, R (&w)[6 + NTR]) {
+__device__ __forceinline__ void prims(const Grid<R> &G, const R *s, size_t idx, int k, R (&w)[6 + NTR]) {
   prims_s<R, NTR>(G, s, G.N, idx, k, w);
 }
 
@@ -577,7 +579,7 @@ __device__ __forceinline__ void recon_outer(int f, int line, Load load, StoreOut
 // SPLIT: threads per cell.
 template <class R, int NTR, int TX, int TY, bool IMM, bool LEARNED = false, bool DECOMP = false, bool TMA = false,
           int SPLIT = 1>
-__global__ void __launch_bounds__(TX *TY *SPLIT, SPLIT > 1 ? 1024 / (TX * TY * SPLIT) : LEARNED ? PU_LEARNED_XY_MIN_BLOCKS : (sizeof(R) == 4 ? PU_XY_MIN_BLOCKS : 512 / (TX * TY))) k_xy(const Grid<R> G, const R *__restrict__ sin, R *__restrict__ txy, const __grid_constant__ XyMaps maps) {
+__global__ void __launch_bounds__(TX *TY *SPLIT, SPLIT > 1 ? 1024 / (TX * TY * SPLIT) : LEARNED ? PU_LEARNED_XY_MIN_BLOCKS : (sizeof(R) == 4 ? PU_XY_MIN_BLOCKS : 512 / (TX * TY))) k_xy(const Grid<R> G, const R *sin, R *txy, const __grid_constant__ XyMaps maps) {
   using Sh = XYShape<R, NTR, TX, TY, IMM, LEARNED>;
   constexpr int F = Sh::F, S = Sh::S, NT = Sh::NT * SPLIT, HX = Sh::HX, HY = Sh::HY, EN = Sh::EN, FN = Sh::FN;
   static_assert(SPLIT == 1 || (sizeof(R) == 4 && !LEARNED), "split positions: the packed limiter");
@@ -1356,8 +1358,8 @@ struct ZtMaps {
 template <class R, int NTR, int TX, int TZ, bool IMM, bool TMA = false, int SPLIT = 1>
 __global__ void __launch_bounds__(TX *TZ *SPLIT,
                                   SPLIT > 1 ? 1 : sizeof(R) == 4 ? PU_ZT_MIN_BLOCKS : PU_ZT_MIN_BLOCKS_F64)
-    k_zt(const Grid<R> G, const R *__restrict__ sin, const R *sn, R *sout, const R *__restrict__ txy, R a_n, R a_dt,
-         int n_enforce, const __grid_constant__ ZtMaps maps) {
+    k_zt(const Grid<R> G, const R *__restrict__ sin, const R *sn, R *sout, const R *txy, R a_n, R a_dt, int n_enforce,
+         const __grid_constant__ ZtMaps maps) {
   static_assert(!TMA || sizeof(R) == 4, "TMA staging: FP32");
   using Sh = ZTShape<R, NTR, TX, TZ, IMM>;
   constexpr int F = Sh::F, S = Sh::S, NT = Sh::NT * SPLIT, HZ = Sh::HZ;
