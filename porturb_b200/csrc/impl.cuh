@@ -308,8 +308,8 @@ struct ImplBase {
     nb = (batch + mlp::TB - 1) / mlp::TB;
     int rc = ml_partials(nb);
     if (rc) return rc;
-    k_mlp_fwd_bwd<<<nb, mlp::TB, mlp::SM_FLOATS * sizeof(float), st>>>(ml_wq, xs, ts, ndata, ml_step, seed, batch,
-                                                                       sequential, ml_partial);
+    launch_early(k_mlp_fwd_bwd, dim3(nb), mlp::TB, mlp::SM_FLOATS * sizeof(float), st, ml_wq, xs, ts, ndata, ml_step, seed,
+                 batch, sequential, ml_partial);
     PU_LAUNCHED();
     return PU_OK;
   }
@@ -332,8 +332,8 @@ struct ImplBase {
       ml_step++;
       const float b1 = 0.9f, b2 = 0.999f;
       const float bc1 = float(1.0 - std::pow(0.9, double(ml_step))), bc2 = float(1.0 - std::pow(0.999, double(ml_step)));
-      k_mlp_update<true><<<ML_UPDATE_BLOCKS, 1024, 0, st>>>(ml_partial, nb, ml_grad, ml_theta, ml_m, ml_v, ml_wq,
-                                                           float(lr), b1, b2, 1e-8f, bc1, bc2);
+      launch_early(k_mlp_update<true>, dim3(ML_UPDATE_BLOCKS), 1024, 0, st, ml_partial, nb, ml_grad, ml_theta, ml_m, ml_v,
+                   ml_wq, float(lr), b1, b2, 1e-8f, bc1, bc2);
       PU_LAUNCHED();
       if (it == 0 || it == steps - 1) {
         float L;

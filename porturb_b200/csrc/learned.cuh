@@ -196,10 +196,11 @@ __device__ __forceinline__ void block_grad(const float *R, float *w_out, float *
 // of per-sample tiles in shared memory, 4 x 8 outputs per lane in registers,
 // the block's samples split over its warps.  One tile buffer serves the three
 // layers in turn, so four blocks fit an SM.  Training at batch 65536: 43 us
-// per step (this kernel and k_mlp_update) against 265 us with one thread per
+// per step (this kernel and k_mlp_update; 39 us when launched to overlap)
+// against 265 us with one thread per
 // parameter walking the block's 256 samples (one block per SM, two
 // shared-memory reads per multiply-add) and three kernels after it.
-static __global__ void __launch_bounds__(mlp::TB, 4) k_mlp_fwd_bwd(const float *__restrict__ wq,
+static __global__ void __launch_bounds__(mlp::TB, 4) k_mlp_fwd_bwd(const float *wq,
                                                                    const float *__restrict__ xs,
                                                                    const float *__restrict__ ts, long ndata, long step,
                                                                    unsigned long long seed, int batch, int sequential,
@@ -207,9 +208,11 @@ static __global__ void __launch_bounds__(mlp::TB, 4) k_mlp_fwd_bwd(const float *
   using namespace mlp;
   extern __shared__ __align__(16) float sm[];
   const int tid = threadIdx.x;
+  next_kernel_may_start();
   const long qb = long(blockIdx.x) * TB + tid;
   const bool live = qb < batch;
   float x[NIN], t[NOUT];
+  // The samples are gathered before the last step's update has to be done.
   {
     const long smp = !live ? 0 : (sequential ? qb : batch_sample(seed, step, qb, ndata));
 #pragma unroll
@@ -217,6 +220,7 @@ static __global__ void __launch_bounds__(mlp::TB, 4) k_mlp_fwd_bwd(const float *
 #pragma unroll
     for (int k = 0; k < NOUT; k++) t[k] = live ? ts[smp * NOUT + k] : 0.f;
   }
+  previous_done();
   for (int p = tid; p < NPARAM; p += TB) {
     const float w = wq[p];
     if (p < OFF_B1) sm[SM_W1T + (p % NIN) * WP + p / NIN] = w;
@@ -367,14 +371,14 @@ static __global__ void __launch_bounds__(mlp::TB, 4) k_mlp_fwd_bwd(const float *
 // ADAM: then the Adam update of the FP32 master parameters and the bfloat16
 // copy the next step reads (the loss slot has none).
 template <bool ADAM>
-__global__ void __launch_bounds__(1024) k_mlp_update(const float *__restrict__ partial, int nblocks,
-                                                     float *__restrict__ grad, float *__restrict__ theta,
-                                                     float *__restrict__ mom, float *__restrict__ var,
-                                                     float *__restrict__ wq, float lr, float b1, float b2, float eps,
-                                                     float bc1, float bc2) {
+__global__ void __launch_bounds__(1024) k_mlp_update(const float *partial, int nblocks, float *grad, float *theta,
+                                                     float *mom, float *var, float *wq, float lr, float b1, float b2,
+                                                     float eps, float bc1, float bc2) {
   __shared__ double sums[32][33];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int p = blockIdx.x * 32 + lane;
+  next_kernel_may_start();
+  previous_done();
   double acc = 0.0;
   if (p <= mlp::NPARAM) {
 #pragma unroll 8
