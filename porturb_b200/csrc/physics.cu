@@ -36,7 +36,6 @@ namespace phys {
 
 constexpr int TX = 32, TY = 8, NT = TX * TY;
 constexpr int HX = TX + 2, HY = TY + 2, HP = HX * HY;   // tile plus one halo cell per side
-constexpr int KC = 16;                                  // levels per block
 constexpr int BC_PRECURSOR = 1, BC_WALL = 2;
 constexpr uint8_t F_EQ1 = 1, F_GT0 = 2, F_LT1 = 4;      // immersed proportion == 1, > 0, < 1
 constexpr int iR = 0, iU = 1, iV = 2, iW = 3, iT = 4, iK = 5;
@@ -290,7 +289,7 @@ __device__ __forceinline__ int slot_of(int p) { return ((p % 3) + 3) % 3; }
 
 template <int ND>
 __global__ void __launch_bounds__(NT, 2) k_les(const Grid G, const In in, const Out out, double dt, double vhx,
-                                               double vhy, double vhz) {
+                                               double vhy, double vhz, int kc) {
   constexpr int F = Les<ND>::F, NF = Les<ND>::NF;
   extern __shared__ __align__(16) unsigned char smem[];
   double *ring = reinterpret_cast<double *>(smem);                        // [3][F][HP]
@@ -300,7 +299,7 @@ __global__ void __launch_bounds__(NT, 2) k_les(const Grid G, const In in, const 
   uint8_t *flag = reinterpret_cast<uint8_t *>(raw + Les<ND>::PRE * HP);   // [3][HP]
   const int tid = threadIdx.x, tj = tid / TX, ti = tid % TX;
   const int i0 = blockIdx.x * TX, j0 = blockIdx.y * TY;
-  const int k0 = blockIdx.z * KC, k1 = min(G.nz, k0 + KC);
+  const int k0 = blockIdx.z * kc, k1 = min(G.nz, k0 + kc);
   const int i = i0 + ti, j = j0 + tj;
   const bool live = i < G.nx && j < G.ny;
   const int oc = (tj + 1) * HX + (ti + 1);   // this column's offset in the halo tile
@@ -742,16 +741,39 @@ int copy_back(pu_physics &h, const pu_state_view *v, double *const (&d)[5 + PU_M
   return PU_OK;
 }
 
+// Levels per block of k_les.  Two blocks fit an SM and a block takes about the
+// time of its levels and 2.5 more (the first planes).  16 levels, unless
+// another chunk count fills whole waves better by more than the estimate is
+// worth (15 %; at 10 % a 512x128x64 grid in one chunk was 3 % slower).  us per
+// call with 16 levels / with this: 128x96x64 153 / 117, 64x64x48 126 / 71,
+// 101x67x53 143 / 106, 32x32x32 122 / 60, 384x384x100 1646 / 1610.
+int les_chunk(const pu_physics_config &c) {
+  const long cols = long((c.nx + TX - 1) / TX) * ((c.ny + TY - 1) / TY), slots = 2 * 148;
+  auto estimate = [&](int kc) { return double((cols * ((c.nz + kc - 1) / kc) + slots - 1) / slots) * (kc + 2.5); };
+  int best = std::min(c.nz, 16);
+  double cost = 0.85 * estimate(best);
+  for (int n = 1; n <= (c.nz + 3) / 4; n++) {
+    const int kc = (c.nz + n - 1) / n;
+    const double t = estimate(kc);
+    if (t < cost) {
+      cost = t;
+      best = kc;
+    }
+  }
+  return best;
+}
+
 template <int ND>
 int launch_les(pu_physics &h, const In &in, const Out &out, double dt) {
   const Grid G = make_grid(h);
   const size_t bytes = Les<ND>::bytes;
   PH_CK(cudaFuncSetAttribute(k_les<ND>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)));
-  dim3 grid((h.cfg.nx + TX - 1) / TX, (h.cfg.ny + TY - 1) / TY, (h.cfg.nz + KC - 1) / KC);
+  const int kc = les_chunk(h.cfg);
+  dim3 grid((h.cfg.nx + TX - 1) / TX, (h.cfg.ny + TY - 1) / TY, (h.cfg.nz + kc - 1) / kc);
   const double vhx = 0.5 * (0.25 * h.cfg.dx * h.cfg.dx / dt), vhy = 0.5 * (0.25 * h.cfg.dy * h.cfg.dy / dt),
                vhz = 0.5 * (0.25 * h.cfg.dz * h.cfg.dz / dt);
   cudaEventRecord(h.e0, h.st);
-  k_les<ND><<<grid, NT, bytes, h.st>>>(G, in, out, dt, vhx, vhy, vhz);
+  k_les<ND><<<grid, NT, bytes, h.st>>>(G, in, out, dt, vhx, vhy, vhz, kc);
   cudaEventRecord(h.e1, h.st);
   PH_CK(cudaGetLastError());
   return PU_OK;
