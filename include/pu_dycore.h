@@ -77,7 +77,7 @@ typedef struct pu_config {
   int weno_mode;                           /* pu_weno_mode */
   int device;                              /* CUDA device ordinal */
   void *stream;                            /* cudaStream_t, or NULL */
-  int z_chunk;                             /* 0: the tiled z kernel (FP32 with weno_all) or the z
+  int z_chunk;                             /* 0: the tiled z kernel (weno_all) or the z
                                               march with its own chunk; > 0: the z march with
                                               this many levels per work item (the same results) */
   int thread_loads;                        /* 0: the stage kernels stage their tiles through TMA

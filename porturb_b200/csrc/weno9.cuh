@@ -19,9 +19,10 @@
 // of these operations is what the limiter costs: ~240 per stencil (both
 // edges) against ~280 for the earlier form (an LDL^T factorisation of each
 // window's TV and separate edge formulas, 118 operations up to the TVs and
-// edge values where this one takes 94; MAP_RATIOS below takes 18 more off), and ~25 distinct constants instead
-// of ~100: the 256x256x128 boundary layer 6.53 -> 6.14 ms per step, the
-// 512x512x128 urban canopy 24.2 -> 22.6 ms, the FP64 build 9 % faster.
+// edge values where this one takes 94; MAP_RATIOS below takes 18 more off),
+// and ~25 distinct constants instead of ~100.  Both together took the
+// 256x256x128 boundary layer from 6.53 to 5.98 ms per step and the 512x512x128
+// urban canopy from 24.2 to 22.2 ms.
 // In FP32 the reciprocals use rcp.approx.ftz; every operand is a normal
 // number there (or t^2 = 0, see MAP_RATIOS): TV_k^2+1e-20 >= 1e-20, the
 // normalisation sums exceed 1e-20 on the branch that divides (the weight sums
