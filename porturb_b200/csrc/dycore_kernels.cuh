@@ -131,6 +131,8 @@ struct Grid {
   // can run its interior tiles while its halos cross, its edge tiles after.
   int k_first, c_first, i_first, j_first;
   int late;   // a k_xy launch independent of the kernel before it (see previous_done)
+  int *stage_word;   // the last stage whose input was published, and
+  int stage_no;      // this launch's stage (see publish_input)
   // Learned WENO weights (kernels instantiated with LEARNED only).
   const uint32_t *ml_frags;     // per-lane operand fragments of the network
   unsigned long long *ml_counts;  // [0] stencils given learned weights, [1] limiter fallbacks
@@ -172,8 +174,8 @@ __device__ __forceinline__ R pow1pm1(const Grid<R> &G, R x) {
 // until the kernel before has completed and its writes are visible (returns at
 // once in a kernel launched the ordinary way).  Every block calls it before it
 // ends, so a kernel that has completed implies that all before it have.
-// What the kernel before writes is read through plain pointers (no
-// __restrict__, no __ldg): a read-only load could be moved ahead of the wait.
+// What an earlier kernel of the chain writes is read through plain pointers
+// (no __restrict__, no __ldg): a read-only load could be moved ahead of the wait.
 //   k_xy  waits first, then lets the z kernel start.  A second k_xy launch of
 //         the same stage (the plain levels after the immersed ones) reads and
 //         writes nothing of the first and waits only at its end (Grid::late):
@@ -181,16 +183,46 @@ __device__ __forceinline__ R pow1pm1(const Grid<R> &G, R x) {
 //   k_zt  forms its fields and reconstructs from the stage input, which was
 //         complete when k_xy let it start, and waits before it reads the x/y
 //         tendency and writes.
+// A kernel's own wait makes the writes of the kernels before it visible to it;
+// letting the next kernel start passes nothing on.  So what k_zt and a late
+// k_xy read ahead of their wait, the stage input, is handed over by a release
+// and an acquire: one thread of the first k_xy launch of a stage publishes the
+// stage's number after its wait (publish_input); a block that reads ahead
+// first looks for its stage's number and waits where it does not find it
+// (input_ready, by one thread; the block's barrier passes it on to the
+// others, the proxy fence to the tile copies).  Two stages that follow one
+// another on a stream never have the same number, replayed graphs included
+// (a graph holds the three stages of a step or a multiple).
+// Blocks that cannot be among the first resident ones start after others have
+// ended, hence after the kernel before: they wait (which returns at once)
+// instead of asking, 0.4 % of the 512x512x128 urban canopy's time.
+// Measured (us per call, all blocks waiting first / this): 64x4x32 one step
+// 68.8 / 62.2, 64x64x48 ten steps 1907 / 1766, 101x67x53 three steps 1495 /
+// 1360, 256x256x128 four steps 23912 / 23866.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void previous_done() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void next_kernel_may_start() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
+// By the last thread of the first block: the first issues the tile copies.
+template <class R>
+__device__ __forceinline__ void publish_input(const Grid<R> &G) {
+  if ((blockIdx.x | blockIdx.y | blockIdx.z) == 0 && threadIdx.x == blockDim.x - 1)
+    asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(G.stage_word), "r"(G.stage_no) : "memory");
+}
+template <class R>
+__device__ __forceinline__ void input_ready(const Grid<R> &G) {
+  int no = G.stage_no - 1;
+  if (blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z) < 148 * 8)   // 256 threads: 8 blocks per SM
+    asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(no) : "l"(G.stage_word) : "memory");
+  if (no != G.stage_no) previous_done();
+  asm volatile("fence.proxy.async.global;" ::: "memory");
+}
 
 template <class R, int NTR>
-__device__ __forceinline__ void load_cell(const Grid<R> &G, const R *__restrict__ s, size_t idx, R (&q)[5 + NTR]) {
+__device__ __forceinline__ void load_cell(const Grid<R> &G, const R *s, size_t idx, R (&q)[5 + NTR]) {
 #pragma unroll
-  for (int v = 0; v < 5 + NTR; v++) q[v] = __ldg(s + v * G.N + idx);
+  for (int v = 0; v < 5 + NTR; v++) q[v] = s[v * G.N + idx];
 }
 
 // Primitive perturbation fields of one cell (dynamics_rk.h:550-558) from its
@@ -607,9 +639,15 @@ __global__ void __launch_bounds__(TX *TY *SPLIT, SPLIT > 1 ? 1024 / (TX * TY * S
   const size_t plane = size_t(k) * G.NP;
   const bool sim2d = G.sim2d != 0;
   if (LEARNED && tid < 2) qn[tid] = 0;
-  if constexpr (LEARNED) load_frags(G.ml_frags, sF, NT);
-  if (!G.late) previous_done();
+  if (G.late) {
+    if (tid == 0) input_ready(G);
+    __syncthreads();
+  } else {
+    previous_done();
+    publish_input(G);
+  }
   next_kernel_may_start();
+  if constexpr (LEARNED) load_frags(G.ml_frags, sF, NT);
 
   // 0. TMA staging of the tile's cross (block-uniform decision).  Box origins:
   // the interior at (i0, j0); the 5 rows above at j0-5 (ny-5 for the first
@@ -1358,7 +1396,7 @@ struct ZtMaps {
 template <class R, int NTR, int TX, int TZ, bool IMM, bool TMA = false, int SPLIT = 1>
 __global__ void __launch_bounds__(TX *TZ *SPLIT,
                                   SPLIT > 1 ? 1 : sizeof(R) == 4 ? PU_ZT_MIN_BLOCKS : PU_ZT_MIN_BLOCKS_F64)
-    k_zt(const Grid<R> G, const R *__restrict__ sin, const R *sn, R *sout, const R *txy, R a_n, R a_dt, int n_enforce,
+    k_zt(const Grid<R> G, const R *sin, const R *sn, R *sout, const R *txy, R a_n, R a_dt, int n_enforce,
          const __grid_constant__ ZtMaps maps) {
   static_assert(!TMA || sizeof(R) == 4, "TMA staging: FP32");
   using Sh = ZTShape<R, NTR, TX, TZ, IMM>;
@@ -1385,10 +1423,14 @@ __global__ void __launch_bounds__(TX *TZ *SPLIT,
   auto src_level = [&](int p) { return (p >= 0 && p < nz) ? p : (wall ? clampi(p, nz) : wrapi(p, nz)); };
 
   next_kernel_may_start();
-  if constexpr (TMA) {
+  if constexpr (!TMA) {
+    if (tid == 0) input_ready(G);
+    __syncthreads();
+  } else {
     if (tid == 0) {
       tma::mbar_init(bar);
       tma::mbar_init(bar + 1);
+      input_ready(G);
       tma::mbar_expect(bar, uint32_t(Sh::raw_bytes));
       tma::load_4d(RAW, &maps.raw, i0, j, k0 - 5, 0, bar);
       if (pref) {

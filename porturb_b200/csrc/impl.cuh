@@ -140,7 +140,8 @@ struct ImplBase {
   void *tabs = nullptr;                       // level tables of type R
   uint8_t *flags = nullptr;
   void *imm_mult = nullptr;
-  int *err = nullptr;
+  int *err = nullptr;    // [0] error bits, [1] the stage kernels' published stage (Grid::stage_word)
+  int stage_no = 0;      // number of the last stage launched
   double *sums = nullptr;
   double *diag_part = nullptr, *diag_out = nullptr;
   int diag_blocks = 0;
@@ -739,8 +740,8 @@ struct Impl : ImplBase {
     lt.rho_e = tb + 5 * nzh;
     lt.theta_e = lt.rho_e + (cfg.nz + 1);
     lt.rt_target = lt.theta_e + (cfg.nz + 1);
-    PU_TRY(dalloc(err, 1));
-    PU_CK(cudaMemsetAsync(err, 0, sizeof(int), st));
+    PU_TRY(dalloc(err, 2));
+    PU_CK(cudaMemsetAsync(err, 0, 2 * sizeof(int), st));
     PU_TRY(dalloc(sums, size_t(3) * cfg.nz));
     diag_blocks = 296;
     PU_TRY(dalloc(diag_part, size_t(diag_blocks) * NDIAG * 2));
@@ -925,6 +926,8 @@ struct Impl : ImplBase {
     G.i_first = 0;
     G.j_first = 0;
     G.late = 0;
+    G.stage_word = err + 1;
+    G.stage_no = stage_no;
     G.ml_frags = ml_frags;
     G.ml_counts = ml_counts;
     G.ml_jump = ml_jump;
@@ -1286,8 +1289,9 @@ struct Impl : ImplBase {
   // One SSPRK3 stage: the x/y kernel (DEC: a decomposed tile reading its
   // received halo slabs), then the z march with the stage combination.
   template <bool IMM, bool LRN, bool DEC = false>
-  int stage(const Grid<R> &G, const R *sin, const R *sn, R *sout, R a_n, R a_dt, int n_enforce) {
+  int stage(Grid<R> G, const R *sin, const R *sn, R *sout, R a_n, R a_dt, int n_enforce) {
     constexpr bool L = LRN && std::is_same<R, float>::value && !DEC;
+    G.stage_no = ++stage_no;
     R *t = static_cast<R *>(txy);
     cudaEvent_t e0 = prof_begin();
     int b = 0;   // sin is s[b]: the tensor maps of that buffer
@@ -1494,7 +1498,7 @@ struct Impl : ImplBase {
   template <bool IMM, int X, int Z>
   int time_step_io(double *const *host, double dt, int nsteps, int nch) {
     NvtxRange range("pu:time_step_overlapped");
-    const Grid<R> G = grid();
+    Grid<R> G = grid();
     R *sb[3] = {static_cast<R *>(s[0]), static_cast<R *>(s[1]), static_cast<R *>(s[2])};
     CouplerPtrs cp;
     CouplerOut co;
@@ -1529,6 +1533,7 @@ struct Impl : ImplBase {
       const R a_n = m == 0 ? R(0) : (m == 1 ? R(3. / 4.) : R(1. / 3.));
       const R a_dt = m == 0 ? R(dt) : (m == 1 ? R(1. / 4. * dt) : R(2. / 3. * dt));
       const int n_enforce = (m == 2 && g != last) ? 2 : 1;
+      G.stage_no = ++stage_no;
       PU_TRY((xy_levels<IMM>(G, sb[m], m, lev(c), lev(c + 1))));
       PU_TRY((zt_chunks<IMM, X, Z>(G, sb[m], m == 0 ? nullptr : sb[0], sb[(m + 1) % 3], a_n, a_dt, n_enforce, m, c,
                                    c + 1)));
@@ -1944,7 +1949,7 @@ struct Impl : ImplBase {
   static size_t scratch_bytes(const pu_config &c) {
     const size_t N = size_t(c.nx) * c.ny * c.nz, nzh = size_t(c.nz) + 2 * HS;
     auto al = [](size_t b) { return (b + 255) / 256 * 256; };
-    return al(sizeof(int)) + al(3 * nzh * sizeof(double)) + al(3 * size_t(c.nz + 1) * sizeof(double)) +
+    return al(2 * sizeof(int)) + al(3 * nzh * sizeof(double)) + al(3 * size_t(c.nz + 1) * sizeof(double)) +
            2 * al(size_t(c.nz) * sizeof(double)) +
            al((5 * nzh + 2 * size_t(c.nz + 1) + size_t(c.nz)) * sizeof(R)) + 4 * al(size_t(5 + NTR) * N * sizeof(R));
   }
@@ -1972,7 +1977,7 @@ struct Impl : ImplBase {
       p += (b + 255) / 256 * 256;
       return q;
     };
-    im.err = reinterpret_cast<int *>(take(sizeof(int)));
+    im.err = reinterpret_cast<int *>(take(2 * sizeof(int)));
     im.cells = reinterpret_cast<double *>(take(3 * size_t(im.nzh) * sizeof(double)));
     im.edges = reinterpret_cast<double *>(take(3 * size_t(c.nz + 1) * sizeof(double)));
     im.rho_off = reinterpret_cast<double *>(take(size_t(c.nz) * sizeof(double)));
@@ -1991,8 +1996,8 @@ struct Impl : ImplBase {
     im.make_maps();
     int rc = im.configure();
     if (rc) return rc;
-    // The array keeps the previous call's contents: the error word must start at zero.
-    PU_CK(cudaMemsetAsync(im.err, 0, sizeof(int), im.st));
+    // The array keeps the previous call's contents: the error and stage words must start at zero.
+    PU_CK(cudaMemsetAsync(im.err, 0, 2 * sizeof(int), im.st));
     const size_t nzh = im.nzh;
     PU_CK(cudaMemcpyAsync(im.cells, dens_cells, nzh * sizeof(double), cudaMemcpyHostToDevice, im.st));
     PU_CK(cudaMemcpyAsync(im.cells + nzh, theta_cells, nzh * sizeof(double), cudaMemcpyHostToDevice, im.st));
