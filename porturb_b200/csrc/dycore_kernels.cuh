@@ -644,7 +644,7 @@ __global__ void __launch_bounds__(TX *TY *SPLIT, SPLIT > 1 ? 1024 / (TX * TY * S
     __syncthreads();
   } else {
     previous_done();
-    publish_input(G);
+    if constexpr (!LEARNED) publish_input(G);   // its z march is launched the ordinary way
   }
   next_kernel_may_start();
   if constexpr (LEARNED) load_frags(G.ml_frags, sF, NT);
@@ -740,6 +740,7 @@ __global__ void __launch_bounds__(TX *TY *SPLIT, SPLIT > 1 ? 1024 / (TX * TY * S
 #pragma unroll
     for (int f = 0; f < F; f++) H[(f * HY + r) * HX + c] = w[f];
   }
+  if constexpr (LEARNED) frags_landed();
   __syncthreads();
   if (IMM) {
     // 1b. The stencil mask of every x and y stencil position, once for all
@@ -1004,11 +1005,16 @@ struct ZShape {
   static constexpr int F = 6 + NTR, NT = TX * TY;
   // 9-plane ring of primitive fields, left edges of the current cell, right
   // edges of the current and the previous cell; all thread-private columns.
-  // Learned mode adds per-warp network scratch and a per-warp fallback queue
-  // of up to F*32 entries.
+  // Learned mode adds the network's fragments and, per warp, network scratch
+  // and a queue of F*32 entries and 32 stencil masks, 16 bits each.
   static constexpr size_t learned_bytes =
-      LEARNED ? size_t(NT / 32) * (mlp::WARP_SMEM_BYTES + F * 32 * 4) + mlp::FRAG_BYTES : 0;
+      LEARNED ? size_t(NT / 32) * (mlp::WARP_SMEM_BYTES + (F + 1) * 32 * 2) + mlp::FRAG_BYTES : 0;
   static constexpr size_t bytes = sizeof(R) * (9 + 3) * size_t(F) * NT + learned_bytes;
+  // Blocks per SM of the learned march: the three its registers allow where
+  // they fit the 228 KB (1 KB of each reserved), up to three tracers.
+  static constexpr int learned_fit = int(228 * 1024 / (bytes + 1024));
+  static constexpr int learned_blocks = learned_fit < PU_LEARNED_Z_MIN_BLOCKS ? learned_fit : PU_LEARNED_Z_MIN_BLOCKS;
+  static_assert(!LEARNED || sizeof(R) != 4 || F > 9 || learned_blocks == PU_LEARNED_Z_MIN_BLOCKS, "three blocks per SM");
 };
 
 // Raw state of one cell (S values) for a later conversion to primitive fields.
@@ -1078,13 +1084,15 @@ __global__ void __launch_bounds__(TX *TY, LEARNED ? PU_LEARNED_Z_MIN_BLOCKS : (s
   R *eR = eL + F * NT;                           // [2][F][NT]
   uint4 *sF = reinterpret_cast<uint4 *>(eR + 2 * F * NT);   // the network's fragments
   uint32_t *sW = reinterpret_cast<uint32_t *>(eR + 2 * F * NT) + mlp::FRAG_BYTES / 4 +
-                 (threadIdx.x >> 5) * ((mlp::WARP_SMEM_BYTES + F * 32 * 4) / 4);
-  uint32_t *wq = sW + mlp::WARP_SMEM_BYTES / 4;  // per-warp fallback queue
+                 (threadIdx.x >> 5) * ((mlp::WARP_SMEM_BYTES + (F + 1) * 32 * 2) / 4);
+  uint16_t *wq = reinterpret_cast<uint16_t *>(sW + mlp::WARP_SMEM_BYTES / 4);   // per-warp queue,
+  uint16_t *wm = wq + F * 32;                                                    // per-lane masks
   unsigned long long n_learned = 0, n_fallback = 0;
   const int tid = threadIdx.x;
   const int i = blockIdx.x * TX + tid % TX, j = blockIdx.y * TY + tid / TX;
   if constexpr (LEARNED) {   // every block is full
     load_frags(G.ml_frags, sF, NT);
+    frags_landed();
     __syncthreads();
   }
   if (i >= G.nx || j >= G.ny) return;            // no block-wide synchronisation below
@@ -1177,9 +1185,14 @@ __global__ void __launch_bounds__(TX *TY, LEARNED ? PU_LEARNED_Z_MIN_BLOCKS : (s
       if constexpr (LEARNED) {
         // The warp's F x 32 stencils, sorted as in recon_learned: the learned
         // ones from the front of the warp's queue, the fallbacks from its back.
+        // An entry is (lane, field); the masks of a lane's stencils, the same
+        // for all fields, lie apart (with them in the entries, 32 bits each, a
+        // third block does not fit an SM at three tracers:
+        // 128x128x64, two steps 4.69 ms against 4.18).
         const int lane = tid & 31, t0 = tid & ~31;
         const unsigned below = (1u << lane) - 1u;
         int nl = 0, cnt = 0;   // the same in every lane
+        wm[lane] = uint16_t(imm | (unsigned(any10) << 9));   // a learned stencil has none
 #pragma unroll 1
         for (int f = 0; f < F; f++) {
           float s[9], x[9];
@@ -1188,21 +1201,24 @@ __global__ void __launch_bounds__(TX *TY, LEARNED ? PU_LEARNED_Z_MIN_BLOCKS : (s
           const float jmp = normalize9(s, x);
           const bool fb = any10 || imm != 0u || jmp > G.ml_jump;
           const unsigned mk = __ballot_sync(0xffffffffu, fb);
-          wq[fb ? F * 32 - 1 - (cnt + __popc(mk & below)) : nl + __popc(~mk & below)] =
-              unsigned(f) | (unsigned(lane) << 4) | (imm << 9) | (unsigned(any10) << 18);
+          wq[fb ? F * 32 - 1 - (cnt + __popc(mk & below)) : nl + __popc(~mk & below)] = uint16_t(f | (lane << 4));
           cnt += __popc(mk);
           nl += __popc(~mk);
         }
         __syncwarp();
         auto load_q = [&](unsigned e, float (&s)[9]) {
-          const int off = t0 - tid + int((e >> 4) & 31u) + int(e & 15u) * NT;
+          const int off = t0 - tid + int(e >> 4) + int(e & 15u) * NT;
 #pragma unroll
           for (int m = 0; m < 9; m++) s[m] = ring[sl[m] + off];
+        };
+        auto load_masked = [&](unsigned e, float (&s)[9], unsigned &mk) {
+          load_q(e, s);
+          mk = wm[e >> 4];
           const int f = int(e & 15u);
-          if (f == iU || f == iV || f == iP) der0_modify(s, (e >> 9) & 511u);
+          if (f == iU || f == iV || f == iP) der0_modify(s, mk & 511u);
         };
         auto store_q = [&](unsigned e, float qL, float qR) {
-          const int o = int(e & 15u) * NT + t0 + int((e >> 4) & 31u);
+          const int o = int(e & 15u) * NT + t0 + int(e >> 4);
           eL[o] = qL;
           eR[par * F * NT + o] = qR;
         };
@@ -1226,14 +1242,15 @@ __global__ void __launch_bounds__(TX *TY, LEARNED ? PU_LEARNED_Z_MIN_BLOCKS : (s
           const bool two = q + half < cnt;
           const unsigned ea = wq[F * 32 - 1 - q], eb = wq[F * 32 - 1 - (two ? q + half : q)];
           float a[9], b[9];
-          load_q(ea, a);
-          load_q(eb, b);
+          unsigned ma, mb;
+          load_masked(ea, a, ma);
+          load_masked(eb, b, mb);
           float2 s2[9], qL, qR;
 #pragma unroll
           for (int m = 0; m < 9; m++) s2[m] = make_float2(a[m], b[m]);
           auto bit = [](unsigned e, int k) { return ((e >> k) & 1u) != 0; };
-          weno9_edges(s2, qL, qR, bool2{!bit(ea, 18), !bit(eb, 18)}, bool2{bit(ea, 12), bit(eb, 12)},
-                      bool2{bit(ea, 14), bit(eb, 14)});
+          weno9_edges(s2, qL, qR, bool2{!bit(ma, 9), !bit(mb, 9)}, bool2{bit(ma, 3), bit(mb, 3)},
+                      bool2{bit(ma, 5), bit(mb, 5)});
           store_q(ea, qL.x, qR.x);
           if (two) store_q(eb, qL.y, qR.y);
         }

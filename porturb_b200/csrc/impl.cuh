@@ -1267,17 +1267,19 @@ struct Impl : ImplBase {
   }
 
   // Levels per chunk of the learned z march, three of whose blocks fit an SM
-  // and all of which take about the time of their levels and 3 more (the two
-  // closing cells, the first planes): the chunk count that fills whole waves
-  // best.  128x128x64 columns in chunks of 16 levels are 512 blocks, 1.15
-  // waves: 398 us per launch, 332 us in three chunks; 64x64x48 195 and 118 us.
+  // (two with four tracers) and all of which take about the time of their
+  // levels and 3 more (the two closing cells, the first planes): the chunk
+  // count that fills whole waves best.  128x128x64 columns in chunks of 16
+  // levels are 512 blocks, 1.15 waves: 398 us per launch, 332 us in three
+  // chunks; 64x64x48 195 and 118 us.  Two steps of 128x128x64 with four
+  // tracers: 5.35 ms with the waves counted at three blocks, 4.89 ms.
   int learned_z_chunk() const {
-    const size_t cols = size_t(cfg.nx / ZTX) * (cfg.ny / ZTY);
+    const size_t cols = size_t(cfg.nx / ZTX) * (cfg.ny / ZTY), slots = 148 * ZShape<R, NTR, ZTX, ZTY, true>::learned_blocks;
     int best = cfg.nz;
     double cost = 1e300;
     for (int c = 1; c <= (cfg.nz + 7) / 8; c++) {
       const int kc = (cfg.nz + c - 1) / c;
-      const double t = double((cols * blocks(cfg.nz, kc) + 3 * 148 - 1) / (3 * 148)) * (kc + 3);
+      const double t = double((cols * blocks(cfg.nz, kc) + slots - 1) / slots) * (kc + 3);
       if (t < cost) {
         cost = t;
         best = kc;

@@ -454,6 +454,7 @@ static __global__ void __launch_bounds__(128) k_mlp_eval_mma(const uint32_t *__r
   uint4 *sF = reinterpret_cast<uint4 *>(smem_raw);
   uint32_t *sW = reinterpret_cast<uint32_t *>(smem_raw + mlp::FRAG_BYTES + warp * mlp::WARP_SMEM_BYTES);
   load_frags(frags, sF, blockDim.x);
+  frags_landed();
   __syncthreads();
   const long q = (long(blockIdx.x) * (blockDim.x >> 5) + warp) * 32 + lane;
   float x[9], wl[5], wr[5];

@@ -128,11 +128,15 @@ static __global__ void k_mlp_frags(const float *__restrict__ theta, uint32_t *__
   put(0u);
 }
 
-// The fragments into shared memory, by the block's nt threads (the caller
-// synchronises).
-__device__ __forceinline__ void load_frags(const uint32_t *__restrict__ frags, uint4 *sF, int nt) {
-  for (int e = threadIdx.x; e < mlp::FRAG_GROUPS * 32; e += nt) sF[e] = __ldg(reinterpret_cast<const uint4 *>(frags) + e);
+// The fragments into shared memory, by asynchronous copies of the block's nt
+// threads; frags_landed waits for a thread's own (the caller synchronises).
+__device__ __forceinline__ void load_frags(const uint32_t *frags, uint4 *sF, int nt) {
+  for (int e = threadIdx.x; e < mlp::FRAG_GROUPS * 32; e += nt)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(sF + e))),
+                 "l"(reinterpret_cast<const uint4 *>(frags) + e)
+                 : "memory");
 }
+__device__ __forceinline__ void frags_landed() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 __device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1,
                                          const float (&c)[4]) {
