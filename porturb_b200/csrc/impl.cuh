@@ -1133,8 +1133,19 @@ struct Impl : ImplBase {
   // The tiled z kernel (k_zt) takes the plain limiter with weno_all, unless a
   // z chunk was asked for (the march; in FP32 it gives the same bits).  Its
   // grid has one y row per block row, so ny is held to the grid's y limit.
+  // FP64 on up to 16 levels keeps the march on many columns: the tile computes
+  // 32 levels' closing cells and fields for them and has more blocks than the
+  // march needs to fill the device.  Two steps, us, tile / march: 96x96x4 449 /
+  // 394, 128x128x6 738 / 615, 128x128x8 827 / 765, 192x192x16 2375 / 2210,
+  // 512x256x4 4262 / 2097, 512x256x16 8179 / 7428; below the line 64x64x4 336 /
+  // 401, 96x96x6 483 / 534, 96x96x8 491 / 603, 128x128x12 971 / 1056,
+  // 128x128x16 1086 / 1276.  A decomposed tile goes by the whole domain, so
+  // that its FP64 bits do not depend on the decomposition.
   bool z_tiled(bool learned) const {
-    return cfg.weno_all && !learned && cfg.z_chunk <= 0 && cfg.ny <= 65535;
+    const bool shallow = std::is_same<R, double>::value && cfg.nz <= 16 &&
+                         size_t(blocks(dc.on ? dc.d.nx_glob : cfg.nx, ZT_X)) * (dc.on ? dc.d.ny_glob : cfg.ny) >
+                             size_t(250) * cfg.nz;
+    return cfg.weno_all && !learned && cfg.z_chunk <= 0 && cfg.ny <= 65535 && !shallow;
   }
 
   // Learned weights replace the nonlinear limiter where it runs on every

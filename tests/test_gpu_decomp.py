@@ -97,6 +97,23 @@ def test_group_equals_undecomposed(gpu_lib, kind, precision):
     assert not np.array_equal(st, st0)
 
 
+def test_shallow_fp64_group_equals_undecomposed(gpu_lib):
+    """FP64 on few levels takes the z march on many columns: each of the four
+    tiles, too small for that by itself, goes by the whole domain."""
+    case = cases.small_mixed(nx=112, ny=96, nz=4, immersed=False)
+    g = Dycore.from_case(case, precision="f64")
+    dt = g.compute_time_step()
+    g.close()
+    st, tr, cells, _ = _whole(case, "f64", dt)
+    grp = decomp.TileGroup(case, 2, 2, precision="f64")
+    grp.init_case(perturbed=False)
+    _load_tiles(grp, cells)
+    grp.advance(dt, NSTEPS)
+    st_g, tr_g = grp.get_conserved()
+    grp.close()
+    assert np.array_equal(st_g, st) and np.array_equal(tr_g, tr)
+
+
 def test_group_time_step_on_coupler_arrays(gpu_lib):
     """pu_dycore_group_time_step: convert, sub-cycle and convert back per tile
     equals the undecomposed time_step."""

@@ -60,6 +60,22 @@ def test_tiled_z_kernel_in_fp64(name, gpu_lib):
         assert np.abs(a - b).max() <= 1e-12 * max(np.abs(b).max(), 1e-300)
 
 
+@pytest.mark.parametrize("nx,ny,nz,bc_z", [(104, 96, 4, "solid_wall"), (96, 83, 4, "periodic"),
+                                           (250, 130, 5, "solid_wall"), (256, 140, 16, "periodic")])
+def test_shallow_fp64_grids_keep_the_march(nx, ny, nz, bc_z, gpu_lib):
+    """FP64 on up to 16 levels and more than 250 nz tiles of 8 columns (the
+    second case is below that: 996 tiles): the march's results, to the last bit
+    where the call takes it."""
+    case = cases.small_mixed(nx=nx, ny=ny, nz=nz, ntr=1, immersed=False, bc_z=bc_z)
+    _, _, g = gpu_run(case, "f64", 0, 0.0)
+    dt = 0.9 * g.compute_time_step()
+    a = gpu_run(case, "f64", 3, dt)
+    b = gpu_run(case, "f64", 3, dt, z_chunk=16)
+    marches = -(-nx // 8) * ny > 250 * nz
+    for x, y in zip(a[:2], b[:2]):
+        assert np.array_equal(x, y) if marches else np.abs(x - y).max() <= 1e-12 * np.abs(y).max()
+
+
 LARGE = {
     "immersed": lambda: cases.small_mixed(nx=72, ny=40, nz=40),
     "three_tracers_partial": lambda: cases.small_mixed(nx=70, ny=41, nz=45, ntr=3, immersed=False),
