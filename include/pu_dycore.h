@@ -262,8 +262,11 @@ int pu_dycore_learned_counts(pu_dycore *h, long long *learned, long long *fallba
 /* Per-kernel timing with CUDA events recorded on the handle's stream around
  * every stencil-kernel launch while enabled (no counterpart in the reference,
  * whose timers are YAKL's, dynamics_rk.h:104-106).  Kinds: 0 = x/y flux
- * kernel, 1 = z flux + stage kernel, 2 = everything else.  Enabling resets
- * the totals; pu_dycore_profile_read synchronizes. */
+ * kernel, 1 = z flux + stage kernel, 2 = the enforcement that opens a step
+ * (in pu_dycore_time_step with the conversion of the coupler arrays, which is
+ * the same kernel; a decomposed tile's is not recorded).  While enabled,
+ * pu_dycore_time_step does not overlap host copies.  Enabling resets the
+ * totals; pu_dycore_profile_read synchronizes. */
 #define PU_PROFILE_KINDS 3
 typedef struct pu_profile {
   double ms[PU_PROFILE_KINDS];

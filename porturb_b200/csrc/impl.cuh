@@ -1452,7 +1452,9 @@ struct Impl : ImplBase {
     if (!io_overlap(v)) {
       CouplerPtrs cp;
       PU_TRY(device_view(v, cp));
+      cudaEvent_t e0 = prof_begin();
       PU_TRY(load_cells<true>(cp, 0, N));
+      prof_end(2, e0);
       PU_TRY(advance_whole(dt, nsteps, true));
       return store_state(v);
     }

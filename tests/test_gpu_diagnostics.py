@@ -67,3 +67,23 @@ def test_closed_domain_conserves(gpu_lib, precision, bound):
     for k, v in drift.items():
         assert v <= bound, (k, v)
     assert d1["kinetic"] > 0
+
+
+@pytest.mark.parametrize("precision", ["f32", "f64"])
+@pytest.mark.parametrize("immersed", [False, True])
+def test_event_profile_has_every_kind(gpu_lib, precision, immersed):
+    """advance and time_step record three x/y and three z intervals per step
+    and the enforcement that opens the call."""
+    case = cases.small_mixed(immersed=immersed)
+    g = Dycore.from_case(case, precision=precision)
+    arrays = [np.ascontiguousarray(a) for a in case.coupler_arrays(perturbed=True)[:5]]
+    tracers = [np.ascontiguousarray(t) for t in case.tracer_data]
+    g.init(*arrays, tracers, np.ascontiguousarray(case.immersed_proportion) if immersed else None)
+    dt = g.compute_time_step()
+    for call, steps in ((lambda: g.advance(dt, 2), 2), (lambda: g.time_step(*arrays, tracers, 2.5 * dt), 3)):
+        g.profile(True)
+        call()
+        p = g.profile_read()
+        assert [p[k][1] for k in ("xy", "z", "other")] == [3 * steps, 3 * steps, 1]
+        assert all(p[k][0] > 0 for k in p)
+    g.close()
