@@ -77,9 +77,11 @@ typedef struct pu_config {
   int weno_mode;                           /* pu_weno_mode */
   int device;                              /* CUDA device ordinal */
   void *stream;                            /* cudaStream_t, or NULL */
-  int z_chunk;                             /* 0: the tiled z kernel (weno_all) or the z
+  int z_chunk;                             /* 0: the tiled z kernel (weno_all; in FP64 on more
+                                              than 16 levels or few columns) or the z
                                               march with its own chunk; > 0: the z march with
-                                              this many levels per work item (the same results) */
+                                              this many levels per work item (the same bits in
+                                              FP32, the same results to rounding in FP64) */
   int thread_loads;                        /* 0: the stage kernels stage their tiles through TMA
                                               where the grid allows it (nx % 4 == 0); 1: every
                                               tile is loaded by the threads (the same results) */
