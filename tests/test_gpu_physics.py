@@ -125,6 +125,23 @@ def test_les_tracer_counts_and_large_changes(oracle_lib, gpu_lib, diffused, stee
     _check("les/%d/%s" % (diffused, steep), got, want, st)
 
 
+@pytest.mark.parametrize("kind", ["plain", "immersed", "precursor", "periodic_z"])
+def test_les_update_adds_to_the_given_values(gpu_lib, kind):
+    """A step too short to change anything returns the coupler arrays bit for
+    bit: the update adds to the values given instead of forming them again from
+    mixing ratios (two more roundings per tracer)."""
+    case, halos, _ = _case(kind, nx=37, ny=19, nz=21)
+    case.tracers = list(case.tracers) + [cases.Tracer("t0", "", False, False, True)]
+    case.tracer_data = np.concatenate([case.tracer_data, np.full((1,) + case.rho_d.shape, 0.3)])
+    st = pyphysics.state_of(case, seed=5)
+    st["tracers"][2] += 0.1 * np.random.default_rng(5).standard_normal(case.rho_d.shape)
+    ph = Physics.from_case(case, halos=halos)
+    got = _run_gpu(ph, "les", st, (1e-200,), True)
+    ph.close()
+    for key in st:
+        assert np.array_equal(got[key], st[key]), key
+
+
 def test_les_out_of_place_equals_in_place(gpu_lib):
     import torch
     case, halos, _ = _case("immersed")
