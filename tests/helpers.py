@@ -1,5 +1,7 @@
 """Shared helpers of the parity tests: run the same case through the CPU
 oracle and through libpu_dycore on identical inputs and compare."""
+import dataclasses
+
 import numpy as np
 
 import pyoracle
@@ -36,6 +38,15 @@ def gpu_run(case, precision, nsteps, dt, hydro=None, **kw):
     g.synchronize()
     st, tr = g.get_conserved()
     return st, tr, g
+
+
+def twice_in_y(case):
+    """The case with its flow repeated once more in y."""
+    rep = lambda a: np.ascontiguousarray(np.concatenate([a, a], axis=-2))
+    pert = None if case.perturbed is None else {k: rep(v) for k, v in case.perturbed.items()}
+    return dataclasses.replace(case, ny=2 * case.ny, ylen=2 * case.ylen, perturbed=pert,
+                               **{f: rep(getattr(case, f)) for f in ("rho_d", "uvel", "vvel", "wvel", "temp",
+                                                                     "tracer_data", "immersed_proportion")})
 
 
 def rel_change_err(a, b, base):

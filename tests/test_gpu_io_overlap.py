@@ -2,7 +2,8 @@
 (pu_config.serial_io = 0) gives the same bits as copies in, steps, copies
 out (serial_io = 1).
 
-The overlapped call runs as a wavefront over chunks of 32 levels: the input
+The overlapped call runs as a wavefront over chunks of 8, 16 or 32 levels
+(Impl::io_levels; 32 on the small grids of the first test): the input
 crosses chunk by chunk on a copy stream, and stage g runs on chunk c once
 stage g-1 has run on chunks c-1, c and c+1 (launches in diagonals g + c),
 each chunk's final state converted back and copied out while the others
@@ -73,33 +74,47 @@ def test_overlapped_time_step_same_bits(name, factor, pinned, gpu_lib):
     assert np.array_equal(st0, st1) and np.array_equal(tr0, tr1)
 
 
+def _check_levels(case, levels, steps, launches):
+    """A call in chunks of that many levels launches the conversion in and out
+    and two stage kernels per stage for every chunk, and a third per stage for
+    a chunk that the immersed levels end in."""
+    chunks = -(-case.nz // levels)
+    assert launches - chunks * (2 + 6 * steps) in ((0, 3 * steps) if case.immersed_proportion.any() else (0,))
+
+
 def test_overlapped_time_step_same_bits_at_config_size(gpu_lib):
     """The urban canopy at the size of its configuration (512x512x128, 2 m:
-    33.5 M cells, 4 chunks, the immersed levels ending inside chunk 1), 3
-    cycles per call from pinned arrays: the same bits both ways."""
+    33.5 M cells, 16 chunks of 8 levels), 3 cycles per call from pinned arrays:
+    the same bits both ways."""
     case = cases.urban_canopy(nx=512, ny=512, nz=128, dx=2.0)
     n1, l1, out1, st1, tr1 = _call(case, True, 2.5, True)
     n0, l0, out0, st0, tr0 = _call(case, False, 2.5, True)
-    assert n0 == n1 == 3 and l0 > l1
+    assert n0 == n1 == 3
+    _check_levels(case, 8, n0, l0)
     for q, (a, b) in enumerate(zip(out0, out1)):
         assert np.array_equal(a, b), (q, np.abs(a - b).max())
     assert np.array_equal(st0, st1) and np.array_equal(tr0, tr1)
 
 
-@pytest.mark.parametrize("name,make,factor", [
-    ("16_levels", lambda: cases.abl_neutral(nx=128, ny=128, nz=66), 1.0),
-    ("16_levels_many_steps", lambda: cases.abl_neutral(nx=144, ny=112, nz=64), 5.0),
-    ("8_levels", lambda: cases.abl_neutral(nx=192, ny=128, nz=70), 2.5),
-    ("8_levels_immersed", lambda: cases.urban_canopy(nx=180, ny=136, nz=73, dx=2.0), 2.5),
+@pytest.mark.parametrize("name,levels,make,factor", [
+    ("32_levels_63_tiles", 32, lambda: cases.abl_neutral(nx=144, ny=112, nz=64), 5.0),
+    ("16_levels", 16, lambda: cases.abl_neutral(nx=128, ny=128, nz=66), 1.0),
+    ("16_levels_many_steps", 16, lambda: cases.abl_neutral(nx=144, ny=128, nz=64), 5.0),
+    ("16_levels_immersed", 16, lambda: cases.urban_canopy(nx=140, ny=132, nz=75, dx=2.0), 2.5),
+    ("16_levels_immersed_ragged", 16, lambda: cases.small_mixed(nx=130, ny=120, nz=66, ntr=3), 5.5),
+    ("8_levels", 8, lambda: cases.abl_neutral(nx=192, ny=128, nz=70), 2.5),
+    ("8_levels_immersed", 8, lambda: cases.urban_canopy(nx=180, ny=136, nz=73, dx=2.0), 2.5),
 ])
-def test_thin_chunks_same_bits(name, make, factor, gpu_lib):
-    """Grids of 63 and more 16x16 tiles run in chunks of 16 or 8 levels (16x16
-    and 32x8 z tiles), with last chunks of 1 to 6 levels: the bits of the
-    serial form."""
+def test_thin_chunks_same_bits(name, levels, make, factor, gpu_lib):
+    """Grids of 64 and more 16x16 tiles run in chunks of 16 or 8 levels (16x16
+    and 32x8 z tiles), one step and several SSPRK3 cycles, with and without
+    immersed cells, with last chunks of 1 to 11 levels: the bits of the serial
+    form."""
     case = make()
     n1, l1, out1, st1, tr1 = _call(case, True, factor, False)
     n0, l0, out0, st0, tr0 = _call(case, False, factor, False)
-    assert n0 == n1 and l0 > l1
+    assert n0 == n1
+    _check_levels(case, levels, n0, l0)
     for q, (a, b) in enumerate(zip(out0, out1)):
         assert np.array_equal(a, b), (name, q, np.abs(a - b).max())
     assert np.array_equal(st0, st1) and np.array_equal(tr0, tr1)

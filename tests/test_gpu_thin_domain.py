@@ -2,23 +2,13 @@
 edges of the halo cells that close a y line from the tile's own first and last
 cells.  The same flow repeated once more in y (ny = 8, two tiles, whose closing
 cells are reconstructed) gives the same bits, on the same profiles."""
-import dataclasses
-
 import numpy as np
 import pytest
 
-from helpers import gpu_run
+from helpers import gpu_run, twice_in_y
 from porturb_b200 import cases
 
 pytestmark = pytest.mark.gpu
-
-
-def _twice(case):
-    rep = lambda a: np.ascontiguousarray(np.concatenate([a, a], axis=-2))
-    pert = None if case.perturbed is None else {k: rep(v) for k, v in case.perturbed.items()}
-    return dataclasses.replace(case, ny=2 * case.ny, ylen=2 * case.ylen, perturbed=pert,
-                               **{f: rep(getattr(case, f)) for f in ("rho_d", "uvel", "vvel", "wvel", "temp",
-                                                                     "tracer_data", "immersed_proportion")})
 
 
 @pytest.mark.parametrize("precision", ["f32", "f64"])
@@ -28,6 +18,6 @@ def test_closing_cells_of_a_thin_periodic_domain(gpu_lib, precision, nx, nz, imm
     _, _, g = gpu_run(case, precision, 0, 0.0)
     dt, cells = 0.9 * g.compute_time_step(), g.get_hydrostasis()[0]
     st4, tr4, _ = gpu_run(case, precision, 3, dt, hydro=cells)
-    st8, tr8, _ = gpu_run(_twice(case), precision, 3, dt, hydro=cells)
+    st8, tr8, _ = gpu_run(twice_in_y(case), precision, 3, dt, hydro=cells)
     for a, b in ((st4, st8), (tr4, tr8)):
         assert np.array_equal(a, b[:, :, :4]) and np.array_equal(a, b[:, :, 4:])

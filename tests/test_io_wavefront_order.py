@@ -4,7 +4,7 @@ every chunk reads the versions of the state buffers that the serial order
 (load_state, then the stages of advance one after the other) gives it, and
 leaves the same final versions.
 
-Model: chunk c of ZT_Z levels; op (0, c) brings chunk c in (writes s0[c]);
+Model: chunk c of 8, 16 or 32 levels (the last one of any number); op (0, c) brings chunk c in (writes s0[c]);
 op (g, c), g = 1 .. 3 nsteps, is stage g on chunk c: stage m = (g-1) % 3
 reads s0 / s1 / s2 at chunks c-1, c, c+1 (the z stencils reach 5 levels into
 each neighbour; the x/y stencils stay in the level) and, for m = 1, 2, s0 at
@@ -48,7 +48,7 @@ def versions(order, nch):
 
 
 @pytest.mark.parametrize("nsteps", [1, 2, 3, 4, 10])
-@pytest.mark.parametrize("nch", [2, 3, 4, 8, 9])
+@pytest.mark.parametrize("nch", [2, 3, 4, 8, 9, 16])
 def test_wavefront_reads_the_serial_versions(nch, nsteps):
     last = 3 * nsteps
     w, s = wavefront(nch, last), serial(nch, last)

@@ -17,7 +17,8 @@ staged tile of every grid here:
 * every cell of the cross comes from the box cell holding the global cell
   the threads' path reads (periodic wrap, precursor clamp).
 
-k_zt's boxes start at (i0, j, k0-5) and (i0, j, k0) with i0 a multiple of 8;
+k_zt's tiles are 8x32, 16x16 or 32x8 (columns x levels); its boxes start at
+(i0, j, k0-5) and (i0, j, k0) with i0 a multiple of the tile's columns;
 a level's row in the halo box is its level minus k0-5, used only inside the
 box (the threads load the rest), so every row it reads holds the level the
 threads' path reads.
@@ -118,17 +119,16 @@ def test_xy_tiles_at_precursor_edges_keep_thread_loads():
     assert xy_boxes(16, 0, nx, ny, PERIODIC, PRECURSOR) is None
 
 
-ZT_X, ZT_Z = 8, 32
-
-
+@pytest.mark.parametrize("zt_x,zt_z", [(8, 32), (16, 16), (32, 8)])
 @pytest.mark.parametrize("nz,wall", [(40, True), (40, False), (64, True), (96, False), (128, True), (20, True)])
 @pytest.mark.parametrize("nx", [8, 20, 64])
-def test_zt_boxes(nx, nz, wall):
-    hz = ZT_Z + 10
-    for k0 in range(0, nz, ZT_Z):
-        for i0 in range(0, nx, ZT_X):
+def test_zt_boxes(nx, nz, wall, zt_x, zt_z):
+    hz = zt_z + 10
+    assert zt_x * zt_z == 256 and zt_x * 4 % 16 == 0     # the copied tile's inner extent
+    for k0 in range(0, nz, zt_z):
+        for i0 in range(0, nx, zt_x):
             assert i0 % 4 == 0
-            for p in range(k0 - 5, k0 + ZT_Z + 5):
+            for p in range(k0 - 5, k0 + zt_z + 5):
                 lv = p if 0 <= p < nz else (clamp(p, nz) if wall else wrap(p, nz))
                 rr = lv - (k0 - 5)
                 if 0 <= rr < hz:
