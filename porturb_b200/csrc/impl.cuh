@@ -1494,6 +1494,13 @@ struct Impl : ImplBase {
   //   192x128x96    2 steps 7.68 / 6.40 / 5.78  4 steps 11.1 / 10.1 / 9.9
   //                 6 steps 14.6 / 13.8 / 14.0
   //   128x128x128   4 steps 9.57 / 8.69 / 8.77  10 steps 18.9 / 18.8 / 20.1
+  // and on grids that the lines below were not drawn from:
+  //   160x112x96 (70 tiles)     1 step 4.44 / 3.83 / 4.16  3 steps 7.07 / 6.22 / 5.87  6 steps 11.0 / 10.4 / 10.5
+  //   144x128x200 (72 tiles)    2 steps 9.55 / 8.17 / 8.91  8 steps 26.4 / 25.7 / 29.3
+  //   208x160x96 (130 tiles)    1 step 8.00 / 6.77 / 7.11  2 steps 10.3 / 8.50 / 7.43  5 steps 17.4 / 15.9 / 15.6
+  //   320x288x64 (360 tiles)    1 step 15.7 / 13.3 / 12.3  3 steps 24.0 / 21.8 / 18.4  9 steps 49.0 / 47.3 / 45.4
+  //   384x384x100 (576 tiles)   2 steps 45.8 / 36.6 / 30.5  10 steps 132 / 123 / 120
+  //   48x48x64 (9 tiles)        10 steps 2.51 / 3.17 / 3.86
   int io_levels(int nsteps) const {
     const unsigned tiles = blocks(cfg.nx, XTX_BIG) * blocks(cfg.ny, XTY_BIG);
     if (tiles < 64) return 32;

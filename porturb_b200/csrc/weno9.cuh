@@ -181,11 +181,12 @@ __device__ __forceinline__ V ideal_of(int k, double scale = 1.) {
 // How many of an edge's five weights are mapped by way of the ratio z = u/t^2,
 //   d + t t^6/(t^6 + 2000 u^3) = d + t/(1 + 2000 z^3),
 // which takes seven multiply-adds and two reciprocals against ten and one.
-// The multiply-add pipe bounds the stencil kernels (79 % busy) and the
-// reciprocals' pipe has room (48 %): on the 256x256x128 boundary layer 0, 2, 3,
-// 4 of five take 24.58, 24.02, 23.94, 24.01 ms for four steps (all five, in a
-// first form of this, were slower than three by 1.5 %).  z is infinite where
-// t = 0, and the weight then the ideal one.
+// The multiply-add pipe is the busiest of the stencil kernels' (79 % in k_xy
+// with none, 77 % with three) and the reciprocals' pipe had room (48 %, now
+// 57-64 %): on the 256x256x128 boundary layer 0, 2, 3, 4 of five take 24.58,
+// 24.02, 23.94, 24.01 ms for four steps (all five, in a first form of this,
+// were slower than three by 1.5 %).  z is infinite where t = 0, and the weight
+// then the ideal one.
 constexpr int MAP_RATIOS = 3;
 template <class V, int SIDE>
 __device__ __forceinline__ V odd_of() {
