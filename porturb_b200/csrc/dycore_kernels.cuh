@@ -210,13 +210,31 @@ __device__ __forceinline__ void publish_input(const Grid<R> &G) {
   if ((blockIdx.x | blockIdx.y | blockIdx.z) == 0 && threadIdx.x == blockDim.x - 1)
     asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(G.stage_word), "r"(G.stage_no) : "memory");
 }
+// Whether the block may be among the first resident ones (256 threads: 8 per SM).
+__device__ __forceinline__ bool may_be_early() {
+  return blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z) < 148 * 8;
+}
+// By the thread that issues the tile copies, or (input_ready_block) by a block.
 template <class R>
 __device__ __forceinline__ void input_ready(const Grid<R> &G) {
-  int no = G.stage_no - 1;
-  if (blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z) < 148 * 8)   // 256 threads: 8 blocks per SM
+  if (may_be_early()) {
+    int no;
     asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(no) : "l"(G.stage_word) : "memory");
-  if (no != G.stage_no) previous_done();
-  asm volatile("fence.proxy.async.global;" ::: "memory");
+    if (no == G.stage_no) {
+      asm volatile("fence.proxy.async.global;" ::: "memory");
+      return;
+    }
+  }
+  previous_done();
+}
+template <class R>
+__device__ __forceinline__ void input_ready_block(const Grid<R> &G) {
+  if (may_be_early()) {
+    if (threadIdx.x == 0) input_ready(G);
+    __syncthreads();
+  } else {
+    previous_done();
+  }
 }
 
 template <class R, int NTR>
@@ -639,9 +657,10 @@ __global__ void __launch_bounds__(TX *TY *SPLIT, SPLIT > 1 ? 1024 / (TX * TY * S
   const size_t plane = size_t(k) * G.NP;
   const bool sim2d = G.sim2d != 0;
   if (LEARNED && tid < 2) qn[tid] = 0;
-  if (G.late) {
-    if (tid == 0) input_ready(G);
-    __syncthreads();
+  // Only the plain levels of an undecomposed domain follow another x/y launch.
+  const bool late = !IMM && !LEARNED && !DECOMP && SPLIT == 1 && G.late;
+  if (late) {
+    input_ready_block(G);
   } else {
     previous_done();
     if constexpr (!LEARNED) publish_input(G);   // its z march is launched the ordinary way
@@ -977,7 +996,7 @@ __global__ void __launch_bounds__(TX *TY *SPLIT, SPLIT > 1 ? 1024 / (TX * TY * S
 #pragma unroll
     for (int s = 0; s < S; s++) txy[s * G.N + idx] = tend[s];
   }
-  if (G.late) previous_done();
+  if (late) previous_done();
 }
 
 // Immersed relaxation toward the hydrostatic state and positivity of
@@ -1441,8 +1460,7 @@ __global__ void __launch_bounds__(TX *TZ *SPLIT,
 
   next_kernel_may_start();
   if constexpr (!TMA) {
-    if (tid == 0) input_ready(G);
-    __syncthreads();
+    input_ready_block(G);
   } else {
     if (tid == 0) {
       tma::mbar_init(bar);
