@@ -803,6 +803,15 @@ struct Impl : ImplBase {
     return PU_OK;
   }
 
+  // KB of the partition that four blocks of that size (1 KB of each reserved),
+  // or as many as fit, take.
+  static constexpr int smem_partition(size_t bytes) {
+    const size_t each = bytes + 1024, most = 228 * 1024, need = (4 * each <= most ? 4 : most / each) * each;
+    for (int kb : {100, 132, 164, 196})
+      if (need <= size_t(kb) * 1024) return kb;
+    return 228;
+  }
+
   // Kernel attributes (no allocation).
   int configure() {
     small_tile = cfg.ny < 16;
@@ -835,10 +844,22 @@ struct Impl : ImplBase {
     if constexpr (std::is_same<R, float>::value) {
       PU_TRY((zt_configure<16, 16>()));
       PU_TRY((zt_configure<32, 8>()));
-      if constexpr (XYShape<R, NTR, XTX_BIG, XTY_BIG, false>::TMA_FITS)
+      if constexpr (XYShape<R, NTR, XTX_BIG, XTY_BIG, false>::TMA_FITS) {
         PU_CK(cudaFuncSetAttribute(k_xy<R, NTR, XTX_BIG, XTY_BIG, false, false, false, true>,
                                    cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    int(XYShape<R, NTR, XTX_BIG, XTY_BIG, false>::tma_bytes)));
+        // The z kernel can start beside this one only where it asks for no
+        // larger shared-memory partition: an SM changes it when idle.  Left to
+        // the sizes of four blocks, two tracers take 196 KB here and 228 in
+        // k_zt; four steps, us, so / with 228 in both: 64x24x32 418 / 311,
+        // 64x18x32 400 / 352, 80x18x32 425 / 362, 256x256x128 unchanged.  (For
+        // every stage kernel instead: FP64 2 % slower, tiles loaded by the
+        // threads up to 6 %, for want of L1.)
+        if (smem_partition(ZTShape<R, NTR, ZT_X, ZT_Z, false>::tma_bytes) >
+            smem_partition(XYShape<R, NTR, XTX_BIG, XTY_BIG, false>::tma_bytes))
+          PU_CK(cudaFuncSetAttribute(k_xy<R, NTR, XTX_BIG, XTY_BIG, false, false, false, true>,
+                                     cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+      }
       PU_CK(cudaFuncSetAttribute(k_xy<R, NTR, LTX, LTY, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  int(XYShape<R, NTR, LTX, LTY, false, true>::bytes)));
       PU_CK(cudaFuncSetAttribute(k_xy<R, NTR, LTX, LTY, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
